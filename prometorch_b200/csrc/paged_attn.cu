@@ -93,6 +93,56 @@ __global__ void __launch_bounds__(256) paged_rope_write_kernel(const __grid_cons
     }
 }
 
+// The same for projections in bf16 with 16-byte rows: a thread rotates eight pairs (two 16-byte loads, D/16 threads a head) or moves eight
+// values.  What bounds it is bytes: each value is read once and written once or twice.  One CTA per token either way; two bytes
+// an access it cost the 8-request, 14192-token prompt pass of a 4096-wide model (8 layers, then 16 tokens each) 88.4 ms in place of 84.2.
+__global__ void __launch_bounds__(256) paged_rope_write_vec_kernel(const __grid_constant__ PagedWriteParams P) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int i = blockIdx.x;
+    const int half = P.D / 2, per_half = half / 8, per_head = P.D / 8;
+    const int pos = P.pos[i];
+    uint4* row = reinterpret_cast<uint4*>(P.qkv + (size_t)i * (P.H + 2 * P.Hk) * P.D);
+    const int page_slot = pos / PAGE, in_page = pos % PAGE;
+    const int page = P.page_table[(size_t)P.req[i] * P.pt_stride + max(0, min(page_slot, P.pt_stride - 1))];
+    const bool ok = pos >= 0 && pos < P.max_pos && page_slot < P.pt_stride && page >= 0 && page < P.n_pages;
+    if (!ok) {
+        if (threadIdx.x == 0 && P.status) atomicExch(P.status, PTB_ERR_BOUNDS);
+        return;
+    }
+    const float4* cs = reinterpret_cast<const float4*>(P.cos + (size_t)pos * half);
+    const float4* sn = reinterpret_cast<const float4*>(P.sin + (size_t)pos * half);
+    auto slot = [&](__nv_bfloat16* pages, int kh) { return reinterpret_cast<uint4*>(pages + (((size_t)page * P.Hk + kh) * PAGE + in_page) * P.D); };
+    const int n_rot = (P.H + P.Hk) * per_half, n_all = n_rot + P.Hk * per_head;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < n_all; e += 256) {
+        if (e < n_rot) {
+            const int h = e / per_half, j = e - h * per_half;
+            const uint4 lo = row[h * per_head + j], hi = row[h * per_head + per_half + j];
+            const float4 c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = sn[2 * j], s1 = sn[2 * j + 1];
+            const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+            const __nv_bfloat162 *a2 = reinterpret_cast<const __nv_bfloat162*>(&lo), *b2 = reinterpret_cast<const __nv_bfloat162*>(&hi);
+            uint4 ra, rb;
+            __nv_bfloat162 *oa = reinterpret_cast<__nv_bfloat162*>(&ra), *ob = reinterpret_cast<__nv_bfloat162*>(&rb);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                const float2 a = __bfloat1622float2(a2[x]), b = __bfloat1622float2(b2[x]);
+                oa[x] = __floats2bfloat162_rn(a.x * c[2 * x] - b.x * s[2 * x], a.y * c[2 * x + 1] - b.y * s[2 * x + 1]);
+                ob[x] = __floats2bfloat162_rn(b.x * c[2 * x] + a.x * s[2 * x], b.y * c[2 * x + 1] + a.y * s[2 * x + 1]);
+            }
+            uint4* dst = h < P.H ? row + h * per_head : slot(P.k_pages, h - P.H);
+            dst[j] = ra; dst[per_half + j] = rb;
+            if (h >= P.H && P.k_out) {
+                uint4* ko = reinterpret_cast<uint4*>(P.k_out + ((size_t)i * P.Hk + h - P.H) * P.D);
+                ko[j] = ra; ko[per_half + j] = rb;
+            }
+        } else {
+            const int c = e - n_rot, kh = c / per_head, d = c - kh * per_head;
+            slot(P.v_pages, kh)[d] = row[(P.H + P.Hk) * per_head + c];
+        }
+    }
+}
+
 struct PagedAttnParams {
     const __nv_bfloat16* q;        // [B, q_stride] with head h at column h * D
     long long q_stride;
@@ -304,7 +354,10 @@ static int rope_write(void* qkv, const float* work, int splits, void* q_out, int
     p.qkv = (__nv_bfloat16*)qkv; p.pos = pos; p.req = req; p.page_table = page_table; p.pt_stride = pt_stride; p.n_pages = n_pages;
     p.cos = cos; p.sin = sin; p.k_pages = (__nv_bfloat16*)k_pages; p.v_pages = (__nv_bfloat16*)v_pages; p.k_out = (__nv_bfloat16*)k_out;
     p.n = n; p.H = H; p.Hk = Hk; p.D = D; p.max_pos = max_pos; p.status = status;
-    PTB_CUDA_OK(ptb_launch(paged_rope_write_kernel, dim3(n), dim3(256), 0, st, ptb_pdl_enabled(), p));
+    // rows of a bf16 projection in 16-byte pieces: half a head is a multiple of eight values and every base is aligned (a head then is too)
+    const bool vec = !work && D % 16 == 0 &&
+                     !(((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)k_out | (uintptr_t)cos | (uintptr_t)sin) & 15);
+    PTB_CUDA_OK(ptb_launch(vec ? paged_rope_write_vec_kernel : paged_rope_write_kernel, dim3(n), dim3(256), 0, st, ptb_pdl_enabled(), p));
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }

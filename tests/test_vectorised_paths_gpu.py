@@ -1,0 +1,27 @@
+"""Wide-access variants of the element-wise kernels at the sizes where they can go wrong, against the tensor-op forms."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,Hk,D,n", [(1, 1, 16, 1), (3, 1, 48, 65), (16, 4, 128, 33), (40, 40, 64, 130), (5, 5, 8, 7)])
+def test_paged_rope_write_rows(H, Hk, D, n):
+    """Head sizes of one and more 16-byte pieces a half (48: three), and 8, which stays with the element-wise kernel: the same pages and rows."""
+    from prometorch_b200.ops import paged as P
+    dev = "cuda"
+    g = torch.Generator(device=dev).manual_seed(H * 100 + n)
+    table = torch.randperm(8, device=dev, generator=g)[:4].int().view(1, 4).contiguous()
+    cos, sin = P.rope_tables(256, D, 10000.0, dev)
+    qkv = torch.randn(n, (H + 2 * Hk) * D, device=dev, generator=g).bfloat16()
+    pos, req = torch.arange(n, dtype=torch.int32, device=dev) + 3, torch.zeros(n, dtype=torch.int32, device=dev)
+    kp = torch.zeros(8, Hk, P.PAGE, D, device=dev, dtype=torch.bfloat16)
+    vp = torch.zeros_like(kp)
+    kr, vr, qr = kp.float().cpu(), vp.float().cpu(), qkv.float().cpu()
+    want = P.paged_rope_write(qr, H, Hk, D, pos.cpu(), req.cpu(), table.cpu(), cos.cpu(), sin.cpu(), kr, vr, want_k=True)
+    k = P.paged_rope_write(qkv, H, Hk, D, pos, req, table, cos, sin, kp, vp, want_k=True)
+    P.check_status(dev)
+    # one rounding to bf16 (2^-9 of a value) over the fp32 result; rotation mixes two values of the pair
+    for a, b in ((k, want), (qkv[:, :H * D], qr[:, :H * D]), (kp, kr)):
+        assert float((a.float().cpu() - b).abs().max()) <= 2 ** -8 * float(b.abs().max())
+    assert torch.equal(vp.float().cpu(), vr)
