@@ -25,3 +25,22 @@ def test_paged_rope_write_rows(H, Hk, D, n):
     for a, b in ((k, want), (qkv[:, :H * D], qr[:, :H * D]), (kp, kr)):
         assert float((a.float().cpu() - b).abs().max()) <= 2 ** -8 * float(b.abs().max())
     assert torch.equal(vp.float().cpu(), vr)
+
+
+@pytest.mark.parametrize("kind", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (15, 512), (16, 256), (17, 2560), (24, 768), (300, 1024)])
+def test_dequant_tiles_of_16_rows(kind, rows, cols):
+    """Rows that end inside a half of eight, one block and several: every value is the file's, rounded once."""
+    from prometorch_b200 import _native as N
+    from prometorch_b200.io import gguf_quant as Q
+    from prometorch_b200.io.gguf_model import pack_weight
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    qt = Q.GGMLType[kind]
+    raw = Q.quantize(torch.randn(rows, cols, device="cuda", generator=g) * 0.02, qt)
+    pw = pack_weight(raw, qt, cols, "cuda", layout=1)
+    out = torch.full((rows + 1, cols), 7.0, dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().ptb_dequant_weight(pw.data.data_ptr(), pw.qtype, 1, rows, cols, out.data_ptr(), torch.cuda.current_stream().cuda_stream), "dequant")
+    want = Q.dequantize(raw, qt, cols).float()
+    # half a step of bf16 (2^-9 of the value), and the fp32 rounding of a difference of two products of the size of the row's largest
+    assert bool(((out[:rows].float() - want).abs() <= want.abs() * 2 ** -8 + 2 ** -21 * want.abs().max()).all())
+    assert bool((out[rows] == 7).all())
