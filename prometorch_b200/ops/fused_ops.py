@@ -28,7 +28,9 @@ def _decls(L):
     L.ptb_gated_act_fwd.argtypes = [vp, vp, ll, ci, ci, ci, vp]
     L.ptb_gated_act_bwd.argtypes = [vp, vp, vp, ll, ci, ci, ci, vp]
     L.ptb_xent.argtypes = [vp, vp, vp, vp, vp, ll, ci, ll, cf, ll, ci, vp]
-    for n in ("ptb_rmsnorm_fwd", "ptb_rmsnorm_bwd", "ptb_rope", "ptb_gated_act_fwd", "ptb_gated_act_bwd", "ptb_xent"):
+    L.ptb_xent_mean.argtypes = [vp, vp, vp, vp, ll, ci, ll, vp, ll, ci, vp]
+    L.ptb_scale_unless_one.argtypes = [vp, ll, vp, ci, vp]
+    for n in ("ptb_rmsnorm_fwd", "ptb_rmsnorm_bwd", "ptb_rope", "ptb_gated_act_fwd", "ptb_gated_act_bwd", "ptb_xent", "ptb_xent_mean", "ptb_scale_unless_one"):
         getattr(L, n).restype = ci
 
 
@@ -238,18 +240,23 @@ class _Xent(torch.autograd.Function):
         dl = None
         if need_grad:
             dl = l2 if inplace else torch.empty_like(l2)
-        # gradient of the MEAN loss is written in the same pass; 1/n_valid is applied in backward
-        N.check(N.lib().ptb_xent(l2.data_ptr(), tgt.data_ptr(), loss.data_ptr(), 0, N.ptr(dl), rows, V, l2.stride(0), 1.0,
-                                 ignore_index, _is_bf16(l2), _stream(logits)), "cross_entropy")
+        # the gradient of the mean loss is written in the same pass
+        N.check(N.lib().ptb_xent_mean(l2.data_ptr(), tgt.data_ptr(), loss.data_ptr(), N.ptr(dl), rows, V, l2.stride(0), n_valid.data_ptr(),
+                                      ignore_index, _is_bf16(l2), _stream(logits)), "cross_entropy")
         if need_grad:
-            ctx.save_for_backward(dl, n_valid)
+            ctx.save_for_backward(dl)
         ctx.shape = logits.shape
         return loss.sum() / n_valid
 
     @staticmethod
     def backward(ctx, g):
-        dl, n_valid = ctx.saved_tensors
-        dl.mul_((g / n_valid).to(dl.dtype))
+        dl, = ctx.saved_tensors
+        if dl.stride(1) == 1 and dl.data_ptr() % 16 == 0 and dl.stride(0) >= dl.shape[1]:      # rows, with the padding between them
+            g = g.float().contiguous()
+            n = (dl.shape[0] - 1) * dl.stride(0) + dl.shape[1] if dl.numel() else 0
+            N.check(N.lib().ptb_scale_unless_one(dl.data_ptr(), n, g.data_ptr(), _is_bf16(dl), _stream(dl)), "cross_entropy_bwd")
+        else:
+            dl.mul_(g.to(dl.dtype))
         return dl.reshape(ctx.shape), None, None, None
 
 

@@ -1,6 +1,7 @@
 """Wide-access variants of the element-wise kernels at the sizes where they can go wrong, against the tensor-op forms."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,22 @@ def test_dequant_tiles_of_16_rows(kind, rows, cols):
     # half a step of bf16 (2^-9 of the value), and the fp32 rounding of a difference of two products of the size of the row's largest
     assert bool(((out[:rows].float() - want).abs() <= want.abs() * 2 ** -8 + 2 ** -21 * want.abs().max()).all())
     assert bool((out[rows] == 7).all())
+
+
+@pytest.mark.parametrize("V,rows", [(1, 3), (8, 1), (65, 33), (520, 7)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("up", [1.0, -2.5])
+def test_cross_entropy_gradient_of_the_mean(V, rows, dtype, up):
+    """Odd widths (padded rows), ignored rows, and an upstream gradient that is not one."""
+    from prometorch_b200.ops.fused_ops import cross_entropy
+    g = torch.Generator(device="cuda").manual_seed(V + rows)
+    x = (torch.randn(rows, V, device="cuda", generator=g) * 2).to(dtype).requires_grad_()
+    t = torch.randint(0, V, (rows,), device="cuda", generator=g)
+    if rows > 2:
+        t[1] = -100
+    (cross_entropy(x, t) * up).backward()
+    r = x.detach().double().requires_grad_()
+    (F.cross_entropy(r, t, ignore_index=-100) * up).backward()
+    # up to two roundings of the stored type, and the fast exponential's error (2^-21 of the largest logit)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -19
+    assert float((x.grad.double() - r.grad).abs().max()) <= 2 * eps * abs(up) / max(1, int((t >= 0).sum()))
