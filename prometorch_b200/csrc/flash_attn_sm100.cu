@@ -1,18 +1,21 @@
-// FlashAttention forward on the 5th-generation tensor cores: both products of every 128 x 128 block run as
+// FlashAttention on the 5th-generation tensor cores: both products of every 128 x 128 block run as
 // tcgen05.mma with accumulators in tensor memory, operands arrive by TMA.
 //
-// One CTA per (128 query rows, head, batch).  Ten warps:
-//   warp 8   TMA producer: the Q tile once, then K and V tiles of 128 keys through two-stage rings;
-//   warp 9   owns tensor memory and issues the MMAs: S(j) = Q K_j^T into one of two 128-column buffers,
-//            then O_j = P_j V_j into a third buffer once the softmax warps have written P_j;
-//   warps 0-7  softmax.  A thread owns one query row (its tensor-memory lane) and half of the block's
-//            columns: it reads its 64 scores with tcgen05.ld, exchanges the row maximum with its partner
-//            thread through shared memory, writes the bf16 probabilities into a 128-byte-swizzled
-//            shared-memory tile (the A operand of the second product) and keeps its half of the output
-//            row in registers, rescaled by the running maximum.  The read-back of O_{j-1} is deferred
-//            until after the scores of block j have been reduced, so that it overlaps the MMA of P_{j-1} V.
+// Forward: one CTA per two tiles of 128 query rows that read the same keys: the same rows of two heads of a group where the
+// group's size is even, else 256 consecutive rows of one head.  Ten warps:
+//   warp 8   TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings;
+//   warp 9   owns tensor memory and issues the MMAs.  Tile t has 128 columns for its scores S_t and D for its output O_t; for every
+//            block j it issues, tile by tile, O_t += P_t(j) V_j and then S_t(j+1) = Q_t K_j+1^T, so that one tile's products run
+//            under the other tile's softmax;
+//   warps 0-3, 4-7   softmax of tile 0 and tile 1.  A thread owns one query row (its tensor-memory lane): it reads the 128 scores
+//            with tcgen05.ld and writes the bf16 probabilities over them (tcgen05.st): they are the A operand of the second product
+//            from tensor memory, and no other thread takes part in a row's maximum or sum.
+// The completion of S_t(j) implies that of O_t's product with block j-1, issued before it, so until P_t(j) is published the softmax
+// warps own O_t too.  They scale it by the change of the running maximum only when some row's maximum has grown by more than a factor
+// 2^8 (weights are then at most 2^8, whose bf16 rounding is as good as that of weights up to 1; sums and outputs are fp32).
 // Causal masking and the sequence end are applied to the blocks that need them only.  Every wait is
-// bounded.  The reference's kernel is aten/src/ATen/cuda/FlashAttention.cu:83-258 (one thread per row).
+// bounded.  Measured (2 x 4001 queries, 32 heads over 8, size 128, causal): 479 us with one tile a CTA, weights through shared memory and
+// outputs in registers, 315 us now (832 TFLOP/s); 4 x 2048, 32 heads over 4, size 64: 245 -> 156 us, bound by the exponentials.  The reference's kernel is aten/src/ATen/cuda/FlashAttention.cu:83-258 (one thread per row).
 #include "gemm_sm100.cuh"
 
 int ptb_make_tmap_bf16(CUtensorMap* map, const void* base, long long inner, long long outer, long long ld, int box_inner, int box_outer);
@@ -27,10 +30,13 @@ constexpr int NTHREADS = 320;
 
 struct Params {
     __nv_bfloat16* O;        // [B, Tq, H, D]
-    float* lse;              // [B, H, Tq] natural-log sum of exponentials
+    float* lse;              // [B, H, Tq] natural-log sum of exponentials, or null
+    const int* cu;           // [B + 1] first row of each sequence in packed q, k and v (then Tq and Tk are read from it), or null
     int B, Tq, Tk, H, Hk;
     int causal, q_offset;
     float scale_log2;        // softmax scale x log2(e)
+    int pair_heads;          // the CTA's tiles are two heads (else two row blocks)
+    int units;               // CTAs per row block: B times heads (pairs of heads)
     int* status;
 };
 
@@ -38,17 +44,32 @@ template <int D>
 struct Sm {
     static constexpr int Q_BYTES = BQ * D * 2;
     static constexpr int KV_BYTES = BKV * D * 2;
-    static constexpr int P_BYTES = BQ * BKV * 2;
     static constexpr int OFF_Q = 0;
-    static constexpr int OFF_K = OFF_Q + Q_BYTES;
+    static constexpr int OFF_K = OFF_Q + 2 * Q_BYTES;
     static constexpr int OFF_V = OFF_K + 2 * KV_BYTES;
-    static constexpr int OFF_P = OFF_V + 2 * KV_BYTES;
-    static constexpr int OFF_RED = OFF_P + P_BYTES;          // 2 x 128 floats
-    static constexpr int OFF_BAR = OFF_RED + 2 * BQ * 4;
+    static constexpr int OFF_BAR = OFF_V + 2 * KV_BYTES;
     static constexpr int TOTAL = OFF_BAR + 256 + 1024;
 };
 
-__device__ __forceinline__ void softmax_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+// D = A B with A (bf16, lane = row, two values of K a column) in tensor memory.
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]),
+        "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]),
+        "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 template <int D>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -60,34 +81,48 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     uint8_t* sq = smem + S::OFF_Q;
     uint8_t* sk = smem + S::OFF_K;
     uint8_t* sv = smem + S::OFF_V;
-    uint8_t* sp = smem + S::OFF_P;
-    float* red = reinterpret_cast<float*>(smem + S::OFF_RED);
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
     uint64_t* q_full = bars;             // [1]
     uint64_t* k_full = bars + 1;         // [2]
     uint64_t* k_empty = bars + 3;        // [2]
     uint64_t* v_full = bars + 5;         // [2]
     uint64_t* v_empty = bars + 7;        // [2]
-    uint64_t* s_full = bars + 9;         // [2]
-    uint64_t* p_ready = bars + 11;       // [1], 8 arrivals (one per softmax warp)
-    uint64_t* o_full = bars + 12;        // [1]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 13);
+    uint64_t* s_full = bars + 9;         // [2] tile t's scores are in tensor memory
+    uint64_t* p_ready = bars + 11;       // [2] tile t's weights are (4 arrivals, one per warp)
+    uint64_t* o_full = bars + 13;        // [2] tile t's output is complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int qb = (int)gridDim.x - 1 - (int)blockIdx.x;           // long (late) query blocks first
-    const int h = blockIdx.y, b = blockIdx.z;
-    const int hk = h / (P.H / P.Hk);
-    const int q0 = qb * BQ;
-    // keys this block can see: [0, kv_end)
-    const int kv_end = P.causal ? min(P.Tk, q0 + BQ + P.q_offset) : P.Tk;
-    const int nblk = max(0, (kv_end + BKV - 1) / BKV);
+    // late row blocks (the long ones under a causal mask) first, over all heads and sequences
+    const int n_rb = (int)gridDim.x / P.units;
+    const int rb = n_rb - 1 - (int)blockIdx.x / P.units, unit = (int)blockIdx.x % P.units;
+    const int per_b = P.units / P.B, b = unit / per_b;
+    const int rows_per = P.pair_heads ? BQ : 2 * BQ;
+    const int h0 = (unit % per_b) * (P.pair_heads ? 2 : 1), hk = h0 / (P.H / P.Hk);
+    int Tq = P.Tq, Tk = P.Tk, qrow = b * P.Tq, krow = b * P.Tk;
+    if (P.cu) {
+        qrow = krow = P.cu[b];
+        Tq = Tk = P.cu[b + 1] - qrow;
+    }
+    const int q0 = rb * rows_per;
+    if (q0 >= Tq) return;                 // a shorter sequence than the longest
+    // blocks of keys that tile t can see
+    auto tile_q0 = [&](int t) { return P.pair_heads ? q0 : q0 + t * BQ; };
+    auto tile_blocks = [&](int t) {
+        const int tq0 = tile_q0(t);
+        if (tq0 >= Tq) return 0;
+        const int end = P.causal ? min(Tk, min(tq0 + BQ, Tq) + P.q_offset) : Tk;
+        return max(0, (end + BKV - 1) / BKV);
+    };
+    const int n0 = tile_blocks(0), n1 = tile_blocks(1), nblk = max(n0, n1);
 
     if (threadIdx.x == 0) {
         mbar_init(q_full, 1);
-        for (int s = 0; s < 2; ++s) { mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1); mbar_init(&s_full[s], 1); }
-        mbar_init(p_ready, 8);
-        mbar_init(o_full, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&k_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_empty[s], 1);
+            mbar_init(&s_full[s], 1); mbar_init(&p_ready[s], 4); mbar_init(&o_full[s], 1);
+        }
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_tmap(&tmQ);
@@ -102,27 +137,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const uint32_t TM_S = 0, TM_O = 256;                           // column offsets: S buffers at 0 and 128, O_j at 256
+    constexpr uint32_t TM_O = 256;                                 // S_t (and P_t over it) at 128 t, O_t at 256 + D t
 
     if (warp == 8) {
         // ---------------------------------------------------------------------------- TMA producer
         if (lane == 0 && nblk > 0) {
             bool ok = true;
-            mbar_expect_tx(q_full, S::Q_BYTES);
-            for (int kb = 0; kb < D / 64; ++kb) tma_load_2d(sq + kb * (BQ * 128), &tmQ, h * D + kb * 64, b * P.Tq + q0, q_full);
+            mbar_expect_tx(q_full, 2 * S::Q_BYTES);
+            for (int t = 0; t < 2; ++t)
+                for (int kb = 0; kb < D / 64; ++kb)
+                    tma_load_2d(sq + t * S::Q_BYTES + kb * (BQ * 128), &tmQ, (h0 + (P.pair_heads ? t : 0)) * D + kb * 64, qrow + tile_q0(t), q_full);
             for (int j = 0; j < nblk && ok; ++j) {
                 const int s = j & 1;
                 if (j >= 2) ok = mbar_wait(&k_empty[s], (uint32_t)(((j >> 1) - 1) & 1), P.status);
                 if (!ok) break;
                 mbar_expect_tx(&k_full[s], S::KV_BYTES);
                 for (int kb = 0; kb < D / 64; ++kb)
-                    tma_load_2d(sk + s * S::KV_BYTES + kb * (BKV * 128), &tmK, hk * D + kb * 64, b * P.Tk + j * BKV, &k_full[s]);
+                    tma_load_2d(sk + s * S::KV_BYTES + kb * (BKV * 128), &tmK, hk * D + kb * 64, krow + j * BKV, &k_full[s]);
                 if (j >= 2) ok = mbar_wait(&v_empty[s], (uint32_t)(((j >> 1) - 1) & 1), P.status);
                 if (!ok) break;
                 mbar_expect_tx(&v_full[s], S::KV_BYTES);
                 for (int hh = 0; hh < 2; ++hh)                       // two halves of 64 keys, each D/64 chunks of [64 keys x 64 dims]
                     for (int c = 0; c < D / 64; ++c)
-                        tma_load_2d(sv + s * S::KV_BYTES + hh * (D / 64) * 8192 + c * 8192, &tmV, hk * D + c * 64, b * P.Tk + j * BKV + hh * 64,
+                        tma_load_2d(sv + s * S::KV_BYTES + hh * (D / 64) * 8192 + c * 8192, &tmV, hk * D + c * 64, krow + j * BKV + hh * 64,
                                     &v_full[s]);
             }
             if (!ok) *abort_flag = 1;
@@ -131,156 +168,175 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         // ---------------------------------------------------------------------------- MMA issuer
         if (lane == 0 && nblk > 0) {
             constexpr uint32_t idesc_s = instr_desc(BQ, BKV, 0, 0);          // S = Q K^T: both K-major
-            constexpr uint32_t idesc_o = instr_desc(BQ, D, 0, 1);            // O = P V: P K-major, V MN-major
-            bool ok = mbar_wait(q_full, 0, P.status);
-            auto issue_s = [&](int j) {
+            constexpr uint32_t idesc_o = instr_desc(BQ, D, 0, 1);            // O = P V: V MN-major
+            auto issue_s = [&](int t, int j) {
                 const int s = j & 1;
-                if (!mbar_wait(&k_full[s], (uint32_t)((j >> 1) & 1), P.status)) return false;
-                tc_fence_after();
-                const uint32_t a0 = smem_u32(sq), b0 = smem_u32(sk + s * S::KV_BYTES);
+                const uint32_t a0 = smem_u32(sq + t * S::Q_BYTES), b0 = smem_u32(sk + s * S::KV_BYTES);
 #pragma unroll
                 for (int kb = 0; kb < D / 64; ++kb)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        umma_bf16(tmem_base + TM_S + (uint32_t)(s * BKV), smem_desc(a0 + kb * (BQ * 128) + k * 32, 16, 1024),
+                        umma_bf16(tmem_base + (uint32_t)(t * BKV), smem_desc(a0 + kb * (BQ * 128) + k * 32, 16, 1024),
                                   smem_desc(b0 + kb * (BKV * 128) + k * 32, 16, 1024), idesc_s, (kb > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&k_empty[s]);
-                umma_commit(&s_full[s]);
-                return true;
+                umma_commit(&s_full[t]);
             };
-            if (ok) ok = issue_s(0);
-            if (ok && nblk > 1) ok = issue_s(1);
+            bool ok = mbar_wait(q_full, 0, P.status) && mbar_wait(&k_full[0], 0, P.status);
+            if (ok) {
+                tc_fence_after();
+                if (n0 > 0) issue_s(0, 0);
+                if (n1 > 0) issue_s(1, 0);
+                umma_commit(&k_empty[0]);
+            }
             for (int j = 0; j < nblk && ok; ++j) {
                 const int s = j & 1;
-                ok = mbar_wait(p_ready, (uint32_t)(j & 1), P.status);        // P_j is in shared memory, O_{j-1} has been read
-                if (ok) ok = mbar_wait(&v_full[s], (uint32_t)((j >> 1) & 1), P.status);
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t a0 = smem_u32(sp), b0 = smem_u32(sv + s * S::KV_BYTES);
+                ok = mbar_wait(&v_full[s], (uint32_t)((j >> 1) & 1), P.status);
+                bool have_k = j + 1 >= nblk;
+                for (int t = 0; t < 2 && ok; ++t) {
+                    const int nt = t ? n1 : n0;
+                    if (j >= nt) continue;
+                    ok = mbar_wait(&p_ready[t], (uint32_t)(j & 1), P.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                    const uint32_t b0 = smem_u32(sv + s * S::KV_BYTES);
 #pragma unroll
-                for (int hh = 0; hh < 2; ++hh)
+                    for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k)
-                        umma_bf16(tmem_base + TM_O, smem_desc(a0 + hh * (BQ * 128) + k * 32, 16, 1024),
-                                  smem_desc(b0 + hh * (D / 64) * 8192 + k * 2048, 8192, 1024), idesc_o, (hh > 0 || k > 0) ? 1u : 0u);
+                        for (int k = 0; k < 4; ++k)
+                            umma_bf16_ts(tmem_base + TM_O + (uint32_t)(t * D), tmem_base + (uint32_t)(t * BKV + (hh * 4 + k) * 8),
+                                         smem_desc(b0 + hh * (D / 64) * 8192 + k * 2048, 8192, 1024), idesc_o, (j > 0 || hh > 0 || k > 0) ? 1u : 0u);
+                    if (j + 1 < nt) {
+                        if (!have_k) {
+                            ok = mbar_wait(&k_full[s ^ 1], (uint32_t)(((j + 1) >> 1) & 1), P.status);
+                            if (!ok) break;
+                            tc_fence_after();
+                            have_k = true;
+                        }
+                        issue_s(t, j + 1);
+                    } else {
+                        umma_commit(&o_full[t]);
+                    }
+                }
                 umma_commit(&v_empty[s]);
-                umma_commit(o_full);
-                if (j + 2 < nblk) ok = issue_s(j + 2);
+                if (j + 1 < nblk) umma_commit(&k_empty[s ^ 1]);
             }
             if (!ok) *abort_flag = 1;
         }
     } else {
         // ---------------------------------------------------------------------------- softmax warps
-        const int row = 32 * (warp & 3) + lane;          // query row inside the block = tensor-memory lane
-        const int hf = warp >> 2;                        // which 64 columns of S, which D/2 columns of O
+        const int t = warp >> 2;                         // tile
+        const int row = 32 * (warp & 3) + lane;          // query row inside the tile = tensor-memory lane
         const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
-        const int q_pos = q0 + row + P.q_offset;         // position of this query among the keys
-        float o_acc[D / 2];
-#pragma unroll
-        for (int i = 0; i < D / 2; ++i) o_acc[i] = 0.f;
-        float m_run = -INFINITY, l_part = 0.f, alpha_prev = 1.f;
+        const uint32_t tm_s = lane_addr + (uint32_t)(t * BKV), tm_o = lane_addr + TM_O + (uint32_t)(t * D);
+        const int tq0 = tile_q0(t), nt = t ? n1 : n0;
+        const int q_pos = tq0 + row + P.q_offset;        // position of this query among the keys
+        float m_run = -INFINITY, l_run = 0.f;
         bool ok = true;
-        auto add_o = [&](float alpha) {                  // o_acc = o_acc * alpha + (my half of the row of O_j)
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-                uint32_t r[32];
-                tmem_ld32(lane_addr + TM_O + (uint32_t)(hf * (D / 2) + c * 32), r);
-                tmem_ld_wait();
-#pragma unroll
-                for (int i = 0; i < 32; ++i) o_acc[c * 32 + i] = o_acc[c * 32 + i] * alpha + __uint_as_float(r[i]);
-            }
-        };
-        for (int j = 0; j < nblk; ++j) {
-            const int s = j & 1;
-            if (ok && !*abort_flag) ok = mbar_wait(&s_full[s], (uint32_t)((j >> 1) & 1), P.status);
+#pragma unroll 1
+        for (int j = 0; j < nt; ++j) {
+            if (ok && !*abort_flag) ok = mbar_wait(&s_full[t], (uint32_t)(j & 1), P.status);
             else ok = false;
             tc_fence_after();
-            float sc[64];
-            {
-                uint32_t r[32];
-                tmem_ld32(lane_addr + TM_S + (uint32_t)(s * BKV + hf * 64), r);
-                tmem_ld_wait();
+            float sc[128];
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sc[i] = __uint_as_float(r[i]) * P.scale_log2;
-                tmem_ld32(lane_addr + TM_S + (uint32_t)(s * BKV + hf * 64 + 32), r);
-                tmem_ld_wait();
+            for (int c = 0; c < 4; ++c) tmem_ld32(tm_s + (uint32_t)(c * 32), reinterpret_cast<uint32_t*>(sc) + c * 32);
+            tmem_ld_wait();
+            float f = P.scale_log2;
+            if (f <= 0.f) {                               // not the usual case: the maximum is that of the scaled scores
 #pragma unroll
-                for (int i = 0; i < 32; ++i) sc[32 + i] = __uint_as_float(r[i]) * P.scale_log2;
+                for (int i = 0; i < 128; ++i) sc[i] *= f;
+                f = 1.f;
             }
-            const int key0 = j * BKV + hf * 64;
-            const bool need_mask = (key0 + 64 > P.Tk) || (P.causal && key0 + 63 > q0 + P.q_offset);
-            if (need_mask) {
+            const int key0 = j * BKV;
+            if ((key0 + BKV > Tk) || (P.causal && key0 + BKV - 1 > tq0 + P.q_offset)) {
+                const int last = P.causal ? min(Tk - 1, q_pos) : Tk - 1;          // last key of this row
 #pragma unroll
-                for (int i = 0; i < 64; ++i) {
-                    const int key = key0 + i;
-                    if (key >= P.Tk || (P.causal && key > q_pos)) sc[i] = -INFINITY;
-                }
+                for (int i = 0; i < 128; ++i)
+                    if (key0 + i > last) sc[i] = -INFINITY;
             }
-            // eight independent partial maxima: a 64-long dependent chain would stall the two warps a scheduler has
             float m8[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) m8[i] = sc[i];
 #pragma unroll
-            for (int i = 8; i < 64; ++i) m8[i & 7] = fmaxf(m8[i & 7], sc[i]);
-            const float mx = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7])));
-            red[hf * BQ + row] = mx;
-            softmax_sync();
-            const float m_blk = fmaxf(red[row], red[BQ + row]);
-            const float m_new = fmaxf(m_run, m_blk);
-            const float m_use = m_new == -INFINITY ? 0.f : m_new;
-            const float alpha = exp2f(m_run - m_use);
+            for (int i = 8; i < 128; ++i) m8[i & 7] = fmaxf(m8[i & 7], sc[i]);
+            const float m_blk = fmaxf(fmaxf(fmaxf(m8[0], m8[1]), fmaxf(m8[2], m8[3])), fmaxf(fmaxf(m8[4], m8[5]), fmaxf(m8[6], m8[7]))) * f;
+            if (__any_sync(0xffffffffu, m_blk > m_run + 8.f)) {
+                const float m_new = fmaxf(m_run, m_blk);
+                const float alpha = m_new == -INFINITY ? 1.f : exp2f(m_run - m_new);
+                m_run = m_new;
+                l_run *= alpha;
+                if (j > 0) {
+#pragma unroll 1
+                    for (int c = 0; c < D / 32; ++c) {
+                        uint32_t r[32];
+                        tmem_ld32(tm_o + (uint32_t)(c * 32), r);
+                        tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+                        tmem_st32(tm_o + (uint32_t)(c * 32), r);
+                    }
+                }
+            }
+            const float m_use = m_run == -INFINITY ? 0.f : m_run;
             float l4[4] = {0.f, 0.f, 0.f, 0.f};
-            uint32_t pk[32];
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float p0 = exp2f(sc[2 * i] - m_use), p1 = exp2f(sc[2 * i + 1] - m_use);
-                l4[i & 3] += p0 + p1;
-                const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
-                pk[i] = *reinterpret_cast<const uint32_t*>(&h2);
-            }
-            l_part = l_part * alpha + ((l4[0] + l4[1]) + (l4[2] + l4[3]));
-            m_run = m_new;
-            // the deferred read-back of O_{j-1}; its MMA ran while the scores above were reduced
-            if (j > 0) {
-                if (ok) ok = mbar_wait(o_full, (uint32_t)((j - 1) & 1), P.status);
-                tc_fence_after();
-                add_o(alpha_prev);
-            }
-            alpha_prev = alpha;
-            // P_j -> shared memory, K-major with the 128-byte swizzle: sub-tile hf, row `row`, 16-byte chunk c at c ^ (row & 7)
-            {
-                uint8_t* prow = sp + hf * (BQ * 128) + row * 128;
+            for (int c = 0; c < 2; ++c) {
+                uint32_t pk[32];
 #pragma unroll
-                for (int c = 0; c < 8; ++c)
-                    *reinterpret_cast<uint4*>(prow + ((c ^ (row & 7)) * 16)) = make_uint4(pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
+                for (int i = 0; i < 32; ++i) {
+                    const float p0 = exp2f(sc[c * 64 + 2 * i] * f - m_use), p1 = exp2f(sc[c * 64 + 2 * i + 1] * f - m_use);
+                    l4[i & 3] += p0 + p1;
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(p0, p1);
+                    pk[i] = *reinterpret_cast<const uint32_t*>(&h2);
+                }
+                tmem_st32(tm_s + (uint32_t)(c * 32), pk);
             }
-            fence_proxy_async();
+            l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+            if (key0 + BKV > Tk) {
+                // rows of V past the end belong to the next sequence: their weights are zero, but zero times what is not finite is not
+                if (ok) ok = mbar_wait(&v_full[j & 1], (uint32_t)((j >> 1) & 1), P.status);
+                if (key0 + row >= Tk && ok) {
+                    uint8_t* vr = sv + (j & 1) * S::KV_BYTES + (row >> 6) * (D / 64) * 8192 + (row & 63) * 128;
+#pragma unroll
+                    for (int i = 0; i < D / 8; ++i) *reinterpret_cast<uint4*>(vr + (i >> 3) * 8192 + (i & 7) * 16) = make_uint4(0, 0, 0, 0);
+                }
+                fence_proxy_async();
+            }
+            tmem_st_wait();
             tc_fence_before();
-            softmax_sync();                   // also keeps `red` from being overwritten before both partners have read it
-            if (lane == 0) mbar_arrive(p_ready);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&p_ready[t]);
         }
-        if (nblk > 0) {
-            if (ok) ok = mbar_wait(o_full, (uint32_t)((nblk - 1) & 1), P.status);
+        if (nt > 0) {
+            if (ok && !*abort_flag) ok = mbar_wait(&o_full[t], 0, P.status);
+            else ok = false;
             tc_fence_after();
-            add_o(alpha_prev);
         }
-        red[hf * BQ + row] = l_part;
-        softmax_sync();
-        const float l = red[row] + red[BQ + row];
-        const int q_idx = q0 + row;
-        if (q_idx < P.Tq && ok) {
-            const float inv = l > 0.f ? 1.0f / l : 0.f;
-            __nv_bfloat16* op = P.O + (((size_t)b * P.Tq + q_idx) * P.H + h) * D + hf * (D / 2);
+        const int q_idx = tq0 + row, h = h0 + (P.pair_heads ? t : 0);
+        const bool valid = q_idx < Tq && ok;
+        const float inv = l_run > 0.f ? 1.0f / l_run : l_run == 0.f ? 0.f : l_run;        // a sum that is not a number stays one
+        __nv_bfloat16* op = P.O + ((size_t)(qrow + q_idx) * P.H + h) * D;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+            uint32_t r[32];
+            if (nt > 0) {
+                tmem_ld32(tm_o + (uint32_t)(c * 32), r);
+                tmem_ld_wait();
+            } else {
 #pragma unroll
-            for (int i = 0; i < D / 2; i += 8) {
-                uint4 o;
-                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(o_acc[i + 2 * e] * inv, o_acc[i + 2 * e + 1] * inv);
-                *reinterpret_cast<uint4*>(op + i) = o;
+                for (int i = 0; i < 32; ++i) r[i] = 0;
             }
-            if (hf == 0) P.lse[((size_t)b * P.H + h) * P.Tq + q_idx] = l > 0.f ? m_run * 0.6931471805599453f + logf(l) : -INFINITY;
+            if (valid) {
+#pragma unroll
+                for (int i = 0; i < 32; i += 8) {
+                    uint4 o;
+                    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) oh[e] = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * e]) * inv, __uint_as_float(r[i + 2 * e + 1]) * inv);
+                    *reinterpret_cast<uint4*>(op + c * 32 + i) = o;
+                }
+            }
         }
+        if (valid && P.lse) P.lse[((size_t)b * P.H + h) * P.Tq + q_idx] = l_run > 0.f ? m_run * 0.6931471805599453f + logf(l_run) : -INFINITY;
         if (!ok) *abort_flag = 1;
     }
     // ---- teardown
@@ -289,23 +345,29 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     if (warp == 9) tmem_dealloc(tmem_base, 512);
 }
 
+// q, k, v: rows of ldq, ldk, ldv elements (heads packed along a row).
 template <int D>
-static int launch(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Tq, int Tk, int H, int Hk, int causal,
-                  float scale, int q_offset, int* status, cudaStream_t st) {
+static int launch(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv, void* o, float* lse, const int* cu, long long rows_q,
+                  long long rows_k, int B, int Tq, int Tk, int H, int Hk, int causal, float scale, int q_offset, int* status, cudaStream_t st) {
+    if (B <= 0 || Tq <= 0 || H <= 0) return 0;
     CUtensorMap mq, mk, mv;
-    if (ptb_make_tmap_bf16(&mq, q, (long long)H * D, (long long)B * Tq, (long long)H * D, 64, BQ)) return -1;
-    if (ptb_make_tmap_bf16(&mk, k, (long long)Hk * D, (long long)B * Tk, (long long)Hk * D, 64, BKV)) return -1;
-    if (ptb_make_tmap_bf16(&mv, v, (long long)Hk * D, (long long)B * Tk, (long long)Hk * D, 64, 64)) return -1;
+    if (ptb_make_tmap_bf16(&mq, q, (long long)H * D, rows_q, ldq, 64, BQ)) return -1;
+    if (ptb_make_tmap_bf16(&mk, k, (long long)Hk * D, rows_k, ldk, 64, BKV)) return -1;
+    if (ptb_make_tmap_bf16(&mv, v, (long long)Hk * D, rows_k, ldv, 64, 64)) return -1;
     static bool attr = false;
     if (!attr) {
         PTB_CUDA_OK(cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sm<D>::TOTAL));
         attr = true;
     }
     Params p;
-    p.O = (__nv_bfloat16*)o; p.lse = lse; p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
+    p.O = (__nv_bfloat16*)o; p.lse = lse; p.cu = cu; p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
     p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-    dim3 grid((Tq + BQ - 1) / BQ, H, B);
-    fwd_kernel<D><<<grid, NTHREADS, Sm<D>::TOTAL, st>>>(mq, mk, mv, p);
+    p.pair_heads = (H / Hk) % 2 == 0;                 // equal lengths side by side; else neighbouring rows, one block apart at most
+    p.units = B * (p.pair_heads ? H / 2 : H);
+    const int rows = p.pair_heads ? BQ : 2 * BQ;
+    const long long ctas = (long long)((Tq + rows - 1) / rows) * p.units;
+    if (ctas > 0x7fffffffLL) { ptb_set_error("flash attention: %lld tiles", ctas); return -1; }
+    fwd_kernel<D><<<(unsigned)ctas, NTHREADS, Sm<D>::TOTAL, st>>>(mq, mk, mv, p);
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }
@@ -627,8 +689,12 @@ PTB_API int ptb_flash_attn_fwd_sm100(const void* q, const void* k, const void* v
         PTB_CUDA_OK(cudaGetDevice(&dev));
         PTB_CUDA_OK(cudaSetDevice(dev));     // the tensor-map encoder is a driver call: bind the primary context to this thread
     }
-    if (D == 128) return ptb::fa100::launch<128>(q, k, v, o, lse, B, Tq, Tk, H, Hk, causal, scale, q_offset, status, st);
-    if (D == 64) return ptb::fa100::launch<64>(q, k, v, o, lse, B, Tq, Tk, H, Hk, causal, scale, q_offset, status, st);
+    auto run = [&](auto f) {
+        return f(q, (long long)H * D, k, (long long)Hk * D, v, (long long)Hk * D, o, lse, nullptr, (long long)B * Tq, (long long)B * Tk, B, Tq, Tk, H, Hk, causal,
+                 scale, q_offset, status, st);
+    };
+    if (D == 128) return run(ptb::fa100::launch<128>);
+    if (D == 64) return run(ptb::fa100::launch<64>);
     ptb_set_error("flash attention (tcgen05): head size %d not supported (64, 128)", D);
     return -1;
 }

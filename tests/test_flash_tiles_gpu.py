@@ -1,0 +1,35 @@
+"""FlashAttention at the edges of its tiles, against plain softmax attention in 64 bits."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+# pairs of heads (even groups) and pairs of row blocks (odd groups); one row, the last block empty, full and ragged; keys that start before
+# the queries, and queries that see none; a second tile past the end
+SHAPES = [(1, 1, 1, 2, 1, 64, True, 0), (1, 127, 127, 2, 2, 128, True, 0), (2, 129, 129, 4, 2, 128, True, 0), (1, 257, 257, 3, 3, 64, True, 0),
+          (2, 256, 384, 6, 2, 64, False, 0), (1, 130, 70, 8, 1, 128, False, 0), (1, 40, 300, 2, 1, 128, True, 260), (1, 200, 64, 3, 1, 128, True, -100),
+          (1, 640, 640, 5, 5, 128, True, 0)]
+
+
+@pytest.mark.parametrize("B,Tq,Tk,H,Hk,D,causal,off", SHAPES)
+@pytest.mark.parametrize("scale", [None, 3.0])
+def test_forward_tiles(B, Tq, Tk, H, Hk, D, causal, off, scale):
+    """``scale`` 3: maxima that keep growing from block to block, so that outputs are scaled on the way."""
+    from prometorch_b200.ops.attention import attention_reference, flash_attention
+    g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
+    q, k, v = (torch.randn(B, t, h, D, device="cuda", generator=g).bfloat16() for t, h in ((Tq, H), (Tk, Hk), (Tk, Hk)))
+    if scale:
+        k = k * torch.linspace(0.1, 1, Tk, device="cuda").bfloat16()[None, :, None, None]
+    o, lse = flash_attention(q, k, v, causal=causal, q_offset=off, scale=scale, return_lse=True)
+    ro, rl = attention_reference(q.double(), k.double(), v.double(), causal, off, scale)
+    seen = torch.isfinite(rl)
+    # weights and outputs are rounded to bf16 once each (2^-9, uniform: 2^-9 / sqrt(3) rms, and fewer than 128 terms dominate a row)
+    assert _rel(o, torch.nan_to_num(ro)) < 4e-3
+    # fp32 sums of 128-term products: 2^-22 of the largest score
+    assert float((lse.double() - rl)[seen].abs().max()) < 1e-4 * max(1.0, float(rl[seen].abs().max()))
+    assert bool((lse[~seen] == float("-inf")).all())
