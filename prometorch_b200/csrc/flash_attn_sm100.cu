@@ -699,6 +699,23 @@ PTB_API int ptb_flash_attn_fwd_sm100(const void* q, const void* k, const void* v
     return -1;
 }
 
+// Sequences of different lengths packed by rows: sequence i has rows cu[i] .. cu[i + 1] (cu: device int [n_seq + 1], rows in all, none longer
+// than max_len) of q, k and v, whose rows are ldq, ldk and ldv elements apart with the heads packed along them; o [rows, H, D].  One launch.
+PTB_API int ptb_flash_attn_varlen_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv, void* o, const int* cu, int n_seq,
+                                      int max_len, long long rows, int H, int Hk, int D, int causal, float scale, int* status, cudaStream_t st) {
+    if (Hk <= 0 || H % Hk) { ptb_set_error("flash attention: %d query heads over %d KV heads", H, Hk); return -1; }
+    if (!cu || rows <= 0 || n_seq <= 0) { ptb_set_error("flash attention: packed sequences need their offsets and at least one row"); return -1; }
+    {
+        int dev = 0;
+        PTB_CUDA_OK(cudaGetDevice(&dev));
+        PTB_CUDA_OK(cudaSetDevice(dev));
+    }
+    if (D == 128) return ptb::fa100::launch<128>(q, ldq, k, ldk, v, ldv, o, nullptr, cu, rows, rows, n_seq, max_len, max_len, H, Hk, causal, scale, 0, status, st);
+    if (D == 64) return ptb::fa100::launch<64>(q, ldq, k, ldk, v, ldv, o, nullptr, cu, rows, rows, n_seq, max_len, max_len, H, Hk, causal, scale, 0, status, st);
+    ptb_set_error("flash attention (tcgen05): head size %d not supported (64, 128)", D);
+    return -1;
+}
+
 extern "C" int ptb_flash_attn_delta(const void* o, const void* dout, float* delta, int B, int Tq, int H, int D, float* dq_zero, cudaStream_t st);
 
 // Backward on tcgen05.  dq: fp32 [B, Tq, H, D] (cleared here, together with the delta pass); delta: fp32 [B, H, Tq] scratch.

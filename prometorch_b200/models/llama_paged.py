@@ -155,33 +155,27 @@ class PagedLlama(PagedModel):
         return self._linear(swiglu(self._linear(x, L["w_gate_up"])), L["w_down"])
 
     def prompt_pass(self, kv, page_table, batch: PromptBatch, hidden: bool = False) -> torch.Tensor:
-        """Attention runs per request over the prompt's own keys (requests of equal length share a call)."""
-        from ..ops.attention import flash_attention
+        """Attention runs over the prompts' own keys, one call for all requests; residual adds go with the norms that follow them."""
+        from ..ops.attention import flash_attention_varlen
+        from ..ops.fused_ops import add_rms_norm
         if any(batch.starts):
             raise ValueError("the Llama prompt pass starts at position 0")
         c, w = self.cfg, self.weights
         H, Hk, Dh = c.num_attention_heads, c.num_key_value_heads, c.head_dim
-        groups: Dict[int, List[int]] = {}
-        for i, n in enumerate(batch.lens()):
-            groups.setdefault(n, []).append(i)
-        consecutive = all(g == list(range(g[0], g[0] + len(g))) for g in groups.values())
         x = w.tok_emb[batch.ids.long()]
+        offs = torch.tensor(batch.offs, dtype=torch.int32, device=x.device)
+        h = self._norm(x, w.layers[0]["attn_norm"]) if w.layers else self._norm(x, w.final_norm)
         for l, L in enumerate(w.layers):
-            qkv = self._linear(self._norm(x, L["attn_norm"]), L["wqkv"]).contiguous()
+            qkv = self._linear(h, L["wqkv"]).contiguous()
             k = P.paged_rope_write(qkv, H, Hk, Dh, batch.pos, batch.req, page_table, self.cos, self.sin, kv.k[l], kv.v[l], want_k=True)
-            a = torch.empty(qkv.shape[0], H * Dh, dtype=qkv.dtype, device=x.device)
-            for n, members in groups.items():
-                runs = [members] if consecutive else [[i] for i in members]      # equal lengths side by side: one call
-                for run in runs:
-                    lo, hi, nb = batch.offs[run[0]], batch.offs[run[-1] + 1], len(run)
-                    q = qkv[lo:hi, :H * Dh].reshape(nb, n, H, Dh)
-                    v = qkv[lo:hi, (H + Hk) * Dh:].reshape(nb, n, Hk, Dh)
-                    a[lo:hi] = flash_attention(q, k[lo:hi].view(nb, n, Hk, Dh), v, causal=True).reshape(nb * n, H * Dh)
-            x = x + self._linear(a, L["wo"])
-            x = x + self._mlp(self._norm(x, L["ffn_norm"]), L)
+            heads = qkv.view(-1, H + 2 * Hk, Dh)
+            a = flash_attention_varlen(heads[:, :H], k, heads[:, H + Hk:], batch.offs, offs).reshape(-1, H * Dh)
+            h, x = add_rms_norm(self._linear(a, L["wo"]), x, L["ffn_norm"], c.rms_norm_eps)
+            nxt = w.layers[l + 1]["attn_norm"] if l + 1 < len(w.layers) else w.final_norm
+            h, x = add_rms_norm(self._mlp(h, L), x, nxt, c.rms_norm_eps)
         if hidden:                                             # the embedding path: every position after the final norm
-            return self._norm(x, w.final_norm)
-        return self._linear(self._norm(x[batch.want], w.final_norm), w.lm_head).float()
+            return h
+        return self._linear(h[batch.want], w.lm_head).float()
 
     def decode_pass(self, kv, page_table, meta: torch.Tensor, nsplit: int) -> torch.Tensor:
         from ..ops.gemm import linear_add_rms_norm, linear_swiglu

@@ -33,6 +33,9 @@ def _decls(L):
     if hasattr(L, "ptb_flash_attn_bwd_sm100"):
         L.ptb_flash_attn_bwd_sm100.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, ci, cf, ci, ci, vp, vp]
         L.ptb_flash_attn_bwd_sm100.restype = ci
+    ll = C.c_longlong
+    L.ptb_flash_attn_varlen_fwd.argtypes = [vp, ll, vp, ll, vp, ll, vp, vp, ci, ci, ll, ci, ci, ci, ci, cf, vp, vp]
+    L.ptb_flash_attn_varlen_fwd.restype = ci
 
 
 def _use_tcgen05() -> bool:
@@ -127,3 +130,24 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, scale: Opti
     else:
         o, lse = attention_reference(q, k, v, causal, q_offset, scale)
     return (o, lse) if return_lse else o
+
+
+def flash_attention_varlen(q, k, v, offs, offs_dev: Optional[torch.Tensor] = None, scale: Optional[float] = None):
+    """Causal attention of packed sequences: sequence i is the rows ``offs[i]:offs[i + 1]`` of ``q [n, H, D]`` and ``k``, ``v [n, Hk, D]``
+    (heads next to one another; rows may be further apart, as in columns of a packed projection).  ``offs`` is a list, ``offs_dev`` the same as an int32
+    tensor on the device.  Returns ``[n, H, D]``.  Inference on a GPU is one launch; otherwise it is :func:`flash_attention` per sequence."""
+    n, H, D = q.shape
+    Hk = k.shape[1]
+    scale = scale if scale is not None else 1.0 / math.sqrt(D)
+    rows_ok = all(t.stride(2) == 1 and t.stride(1) == D and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] * D and t.data_ptr() % 16 == 0 for t in (q, k, v))
+    same = all(t.dtype == torch.bfloat16 and t.is_cuda for t in (q, k, v))
+    grad = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))
+    if n and same and rows_ok and not grad and D in (64, 128) and H % Hk == 0 and offs_dev is not None and _use_tcgen05():
+        from .gemm import _status
+        out = torch.empty(n, H, D, dtype=q.dtype, device=q.device)
+        st = torch.cuda.current_stream(q.device).cuda_stream
+        N.check(N.lib().ptb_flash_attn_varlen_fwd(q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0), out.data_ptr(), offs_dev.data_ptr(),
+                                                  len(offs) - 1, max(b - a for a, b in zip(offs, offs[1:])), n, H, Hk, D, 1, scale,
+                                                  _status(q.device).data_ptr(), st), "flash_attn_varlen")
+        return out
+    return torch.cat([flash_attention(q[a:b][None], k[a:b][None], v[a:b][None], causal=True, scale=scale)[0] for a, b in zip(offs, offs[1:])])

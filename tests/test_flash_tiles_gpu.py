@@ -33,3 +33,26 @@ def test_forward_tiles(B, Tq, Tk, H, Hk, D, causal, off, scale):
     # fp32 sums of 128-term products: 2^-22 of the largest score
     assert float((lse.double() - rl)[seen].abs().max()) < 1e-4 * max(1.0, float(rl[seen].abs().max()))
     assert bool((lse[~seen] == float("-inf")).all())
+
+
+@pytest.mark.parametrize("lens,H,Hk,D", [([1], 1, 1, 64), ([5, 128, 1, 300, 129], 8, 2, 128), ([256, 31, 257], 3, 3, 64), ([127, 64], 4, 4, 128)])
+@pytest.mark.parametrize("packed", [True, False])
+def test_packed_sequences(lens, H, Hk, D, packed):
+    """One launch over sequences side by side, from a packed projection's columns or from tensors of their own; what is not finite in one stays in it."""
+    from prometorch_b200.ops.attention import attention_reference, flash_attention_varlen
+    g = torch.Generator(device="cuda").manual_seed(sum(lens))
+    offs = [0]
+    for n in lens:
+        offs.append(offs[-1] + n)
+    x = torch.randn(offs[-1], H + 2 * Hk, D, device="cuda", generator=g).bfloat16()
+    if len(lens) > 2:
+        x[offs[1]:offs[2]] = float("inf")
+    q, k, v = x[:, :H], x[:, H:H + Hk], x[:, H + Hk:]
+    if not packed:
+        q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
+    o = flash_attention_varlen(q, k, v, offs, torch.tensor(offs, dtype=torch.int32, device="cuda"))
+    for i, (a, b) in enumerate(zip(offs, offs[1:])):
+        if len(lens) > 2 and i == 1:
+            continue
+        want = attention_reference(q[None, a:b].double(), k[None, a:b].double(), v[None, a:b].double(), True)[0][0]
+        assert _rel(o[a:b], want) < 4e-3, i
