@@ -19,6 +19,7 @@
 #include "gemm_sm100.cuh"
 
 int ptb_make_tmap_bf16(CUtensorMap* map, const void* base, long long inner, long long outer, long long ld, int box_inner, int box_outer);
+int ptb_make_tmap_f32_3d(CUtensorMap* map, const void* base, long long n0, long long n1, long long n2, int b0, int b1);
 
 namespace ptb {
 namespace fa100 {
@@ -375,19 +376,25 @@ static int launch(const void* q, long long ldq, const void* k, long long ldk, co
 
 // ---------------------------------------------------------------------------------------------- backward
 // One CTA per (128 keys, KV head, batch); it keeps K_j and V_j in shared memory and dK_j, dV_j in tensor memory, and
-// walks the query blocks that see those keys (all query heads of the KV head's group).  Per query block i:
-//   S = Q_i K_j^T and dP = dO_i V_j^T               two tcgen05.mma groups into TMEM (128 columns each)
-//   P = exp2(S c - lse_i),  dS = P (dP - delta_i) scale   by the thread that owns the query row (= TMEM lane)
-//   dV_j += P^T dO_i,  dK_j += dS^T Q_i,  dQ_i = dS K_j   three groups; dQ_i lands in S's columns, is read back
-//                                                       and added to the fp32 dQ in global memory (vector red)
+// walks the query blocks that see those keys (all query heads of the KV head's group).  The scores are held transposed, a
+// tensor-memory lane per key, so that P^T is the A operand of dV from tensor memory.  Per query block i, in the order of issue:
+//   dV_j += P^T dO_i     P^T = exp2(S^T c - lse_i) in bf16, written by the compute warps over S^T
+//   dP^T = V_j dO_i^T
+//   S^T  = K_j Q_i+1^T   the next block's scores
+//   dK_j += dS^T Q_i     dS^T = P^T (dP^T - delta_i) scale in bf16, in shared memory
+//   dQ_i = dS K_j        lands in dP's columns (head size 128) or its own (64)
+// so the exponentials of block i+1 run under dK and dQ of block i, dS under the next scores, and dQ's read-out under the next dV.
+// With all five products of a block in one chain behind its exponentials the tensor pipe idled more than half of the time
+// (2 x 4001 queries, 32 heads over 8, size 128, causal: 1.70 ms; now 0.95 ms, 690 TFLOP/s; 4 x 2048, 32 heads over 4, size 64: 0.73 -> 0.48 ms).
 // Every tile lives in shared memory in ONE layout, [64-column chunk][row][128 B, 128-byte swizzle], which the
-// descriptors read as a K-major operand (rows = M or N) or as an MN-major operand (rows = K): Q_i is the A operand
-// of S and the B operand of dK, dO_i the A operand of dP and the B operand of dV, K_j the B operand of S and of dQ,
-// and the P / dS tiles written by the threads are A operands in both orientations.
+// descriptors read as a K-major operand (rows = M or N) or as an MN-major operand (rows = K): Q_i is the B operand
+// of S^T and of dK, dO_i that of dP^T and of dV, K_j the A operand of S^T and the B operand of dQ, and dS^T
+// an A operand in both orientations.  dQ_i is added to the fp32 dQ by TMA reductions of 128 x 32 pieces from shared memory: whole
+// lines, where one thread per row added 16 bytes at a time.
+// Sixteen warps: 0-7 compute (a thread has one key and 64 of the block's queries), 8 TMA producer, 9 MMA issuer, 12-15 dQ.
 struct BwdParams {
     const float* lse;        // [B, H, Tq] natural log
     const float* delta;      // [B, H, Tq]
-    float* dq;               // [B, Tq, H, D] fp32, zero-initialised
     __nv_bfloat16* dk;       // [B, Tk, Hk, D]
     __nv_bfloat16* dv;
     int B, Tq, Tk, H, Hk;
@@ -397,50 +404,72 @@ struct BwdParams {
     int gsplit;              // CTAs per KV head: each takes group / gsplit query heads and writes its own dk / dv slice
 };
 
+constexpr int BWD_THREADS = 512;
+// Registers a thread of the compute, dQ and other warps: the launch's 512 x 128 shared out anew (256 x 144 + 128 x 176 + 128 x 48 = 65536).
+constexpr int REGS_COMPUTE = 144, REGS_DQ = 176, REGS_OTHER = 48;
+template <int R> __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(R)); }
+template <int R> __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(R)); }
+
 template <int D>
 struct SmB {
     static constexpr int TILE = 128 * D * 2;                 // K, V, Q, dO
-    static constexpr int PT = 128 * 128 * 2;                 // P, dS
-    static constexpr int NST = D == 64 ? 2 : 1;              // Q_i / dO_i stages: two where shared memory allows
+    static constexpr int PT = 128 * 128 * 2;                 // dS
+    static constexpr int STG = 128 * 32 * 4;                 // a piece of dQ
+    static constexpr int NDO = D == 64 ? 2 : 1;              // dO stages: two where shared memory allows (a block's dO is free again well before the next is needed)
     static constexpr int OFF_K = 0;
     static constexpr int OFF_V = OFF_K + TILE;
     static constexpr int OFF_Q = OFF_V + TILE;
-    static constexpr int OFF_DO = OFF_Q + NST * TILE;
-    static constexpr int OFF_P = OFF_DO + NST * TILE;
-    static constexpr int OFF_DS = OFF_P + PT;
-    static constexpr int OFF_BAR = OFF_DS + PT;
-    static constexpr int TOTAL = OFF_BAR + 256 + 1024;
+    static constexpr int OFF_DO = OFF_Q + 2 * TILE;
+    static constexpr int OFF_DS = OFF_DO + NDO * TILE;
+    static constexpr int OFF_STG = OFF_DS + PT;
+    static constexpr int OFF_ROW = OFF_STG + 2 * STG;        // lse and delta of two query blocks
+    static constexpr int OFF_BAR = OFF_ROW + 2 * 2 * 128 * 4;
+    static constexpr int TOTAL = OFF_BAR + 192;
+    static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
-__device__ __forceinline__ void red_add_v4(float* p, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
+__device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
+    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1),
+                 "r"(c2)
+                 : "memory");
 }
+__device__ __forceinline__ void compute_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ void dq_sync() { asm volatile("bar.sync 2, 128;" ::: "memory"); }
 
 template <int D>
-__global__ void __launch_bounds__(NTHREADS, 1)
+__global__ void __launch_bounds__(BWD_THREADS, 1)
 bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
-           const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ BwdParams P) {
+           const __grid_constant__ CUtensorMap tmDO, const __grid_constant__ CUtensorMap tmDQ, const __grid_constant__ BwdParams P) {
     using S = SmB<D>;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* sk = smem + S::OFF_K;
     uint8_t* sv = smem + S::OFF_V;
     uint8_t* sq = smem + S::OFF_Q;
     uint8_t* sdo = smem + S::OFF_DO;
-    uint8_t* sp = smem + S::OFF_P;
     uint8_t* sds = smem + S::OFF_DS;
+    uint8_t* stg = smem + S::OFF_STG;
+    float* srow = reinterpret_cast<float*>(smem + S::OFF_ROW);       // [block & 1][lse, delta][128]
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + S::OFF_BAR);
-    constexpr int NST = S::NST;
+    constexpr int NDO = S::NDO;
     uint64_t* kv_full = bars;            // K_j, V_j loaded (once)
-    uint64_t* qdo_full = bars + 1;       // [2] Q_i, dO_i loaded
-    uint64_t* qdo_empty = bars + 3;      // [2] the MMAs that read them have completed
-    uint64_t* sdp_full = bars + 5;       // S and dP are in TMEM
-    uint64_t* pds_ready = bars + 6;      // P and dS are in shared memory (8 arrivals)
-    uint64_t* dq_full = bars + 7;        // dV, dK updated, dQ_i in TMEM
-    uint64_t* dq_read = bars + 8;        // dQ_i has been read back (8 arrivals)
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
+    uint64_t* q_full = bars + 1;         // [2] Q_i loaded
+    uint64_t* q_empty = bars + 3;        // [2] the MMAs that read it have completed
+    uint64_t* do_full = bars + 5;        // [2] dO_i loaded
+    uint64_t* do_empty = bars + 7;       // [2]
+    uint64_t* s_full = bars + 9;         // S^T is in TMEM
+    uint64_t* dp_full = bars + 10;       // dP^T is in TMEM
+    uint64_t* p_ready = bars + 11;       // P^T is in TMEM (8 arrivals)
+    uint64_t* ds_ready = bars + 12;      // dS^T is in shared memory (8 arrivals)
+    uint64_t* dq_full = bars + 13;       // dK updated, dQ_i in TMEM
+    uint64_t* dq_read = bars + 14;       // dQ_i has been read back (4 arrivals)
+    uint64_t* all_done = bars + 15;      // dK and dV are complete
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
+    if (smem_u32(smem) & 1023) {         // the swizzled tiles need it, and there is no room to align by hand
+        if (threadIdx.x == 0 && P.status) atomicExch(P.status, PTB_ERR_BOUNDS);
+        return;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int jb = blockIdx.x, hk = blockIdx.y / P.gsplit, part = blockIdx.y % P.gsplit, b = blockIdx.z;
     const int group = (P.H / P.Hk) / P.gsplit;          // query heads this CTA walks
@@ -453,12 +482,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     const int n_it = per_head * group;
 
     if (threadIdx.x == 0) {
-        mbar_init(kv_full, 1); mbar_init(sdp_full, 1);
-        for (int st = 0; st < 2; ++st) { mbar_init(&qdo_full[st], 1); mbar_init(&qdo_empty[st], 1); }
-        mbar_init(pds_ready, 8); mbar_init(dq_full, 1); mbar_init(dq_read, 8);
+        mbar_init(kv_full, 1);
+        for (int st = 0; st < 2; ++st) { mbar_init(&q_full[st], 1); mbar_init(&q_empty[st], 1); mbar_init(&do_full[st], 1); mbar_init(&do_empty[st], 1); }
+        mbar_init(s_full, 1); mbar_init(dp_full, 1); mbar_init(p_ready, 8); mbar_init(ds_ready, 8);
+        mbar_init(dq_full, 1); mbar_init(dq_read, 4); mbar_init(all_done, 1);
         *abort_flag = 0;
         mbar_fence_init();
-        prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO);
+        prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO); prefetch_tmap(&tmDQ);
     }
     if (warp == 9) {
         tmem_alloc(tmem_slot, 512);
@@ -468,11 +498,13 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = 256 + D;      // dQ_i reuses S's columns
+    // P^T over S^T: the weights of queries 0-63 in columns 0-31, of 64-127 in 64-95 (each half over the scores that its own thread has read)
+    constexpr uint32_t TM_S = 0, TM_DP = 128, TM_DV = 256, TM_DK = 256 + D, TM_DQ = D == 64 ? 384 : TM_DP;
 
-    if (warp == 8) {
-        // ---------------------------------------------------------------------------- TMA producer
-        if (lane == 0 && n_it > 0) {
+    if (warp >= 8 && warp < 12) {
+        regs_dec<REGS_OTHER>();
+        if (warp == 8 && lane == 0 && n_it > 0) {
+            // ------------------------------------------------------------------------ TMA producer
             bool ok = true;
             mbar_expect_tx(kv_full, 2 * S::TILE);
             for (int c = 0; c < D / 64; ++c) {
@@ -481,142 +513,219 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             }
             for (int it = 0; it < n_it && ok; ++it) {
                 const int h = head0 + it / per_head, i = i_start + it % per_head;
-                const int stg = it % NST;
-                if (it >= NST) ok = mbar_wait(&qdo_empty[stg], (uint32_t)(((it / NST) - 1) & 1), P.status);
+                const int qs = it & 1, ds = it % NDO;
+                if (it >= 2) ok = mbar_wait(&q_empty[qs], (uint32_t)(((it >> 1) - 1) & 1), P.status);
                 if (!ok) break;
-                mbar_expect_tx(&qdo_full[stg], 2 * S::TILE);
-                for (int c = 0; c < D / 64; ++c) {
-                    tma_load_2d(sq + stg * S::TILE + c * 16384, &tmQ, h * D + c * 64, b * P.Tq + i * 128, &qdo_full[stg]);
-                    tma_load_2d(sdo + stg * S::TILE + c * 16384, &tmDO, h * D + c * 64, b * P.Tq + i * 128, &qdo_full[stg]);
-                }
+                mbar_expect_tx(&q_full[qs], S::TILE);
+                for (int c = 0; c < D / 64; ++c) tma_load_2d(sq + qs * S::TILE + c * 16384, &tmQ, h * D + c * 64, b * P.Tq + i * 128, &q_full[qs]);
+                if (it >= NDO) ok = mbar_wait(&do_empty[ds], (uint32_t)(((it / NDO) - 1) & 1), P.status);
+                if (!ok) break;
+                mbar_expect_tx(&do_full[ds], S::TILE);
+                for (int c = 0; c < D / 64; ++c) tma_load_2d(sdo + ds * S::TILE + c * 16384, &tmDO, h * D + c * 64, b * P.Tq + i * 128, &do_full[ds]);
             }
             if (!ok) *abort_flag = 1;
-        }
-    } else if (warp == 9) {
-        // ---------------------------------------------------------------------------- MMA issuer
-        if (lane == 0 && n_it > 0) {
-            constexpr uint32_t idesc_qk = instr_desc(128, 128, 0, 0);      // S, dP: A [q, D] and B [keys, D] both K-major
-            constexpr uint32_t idesc_tt = instr_desc(128, D, 1, 1);        // dV, dK: A = P / dS read MN-major, B = dO / Q MN-major
-            constexpr uint32_t idesc_dq = instr_desc(128, D, 0, 1);        // dQ: A = dS K-major, B = K MN-major
-            bool ok = mbar_wait(kv_full, 0, P.status);
-            const uint32_t aK = smem_u32(sk), aV = smem_u32(sv), aP = smem_u32(sp), aDS = smem_u32(sds);
-            for (int it = 0; it < n_it && ok; ++it) {
-                const int stg = it % NST;
-                const uint32_t aQ = smem_u32(sq + stg * S::TILE), aDO = smem_u32(sdo + stg * S::TILE);
-                ok = mbar_wait(&qdo_full[stg], (uint32_t)((it / NST) & 1), P.status);
-                if (ok && it > 0) ok = mbar_wait(dq_read, (uint32_t)((it - 1) & 1), P.status);
-                if (!ok) break;
+        } else if (warp == 9 && lane == 0 && n_it > 0) {
+            // ------------------------------------------------------------------------ MMA issuer
+            constexpr uint32_t idesc_t = instr_desc(128, 128, 0, 0);       // S^T, dP^T: both operands K-major
+            constexpr uint32_t idesc_k = instr_desc(128, D, 0, 1);         // dV, dK: A with the queries along K, B = dO / Q MN-major
+            constexpr uint32_t idesc_q = instr_desc(128, D, 1, 1);         // dQ: A = dS^T read MN-major, B = K MN-major
+            const uint32_t aK = smem_u32(sk), aV = smem_u32(sv), aDS = smem_u32(sds);
+            auto issue_s = [&](int it) {
+                const uint32_t aQ = smem_u32(sq + (it & 1) * S::TILE);
+                if (!mbar_wait(&q_full[it & 1], (uint32_t)((it >> 1) & 1), P.status)) return false;
                 tc_fence_after();
 #pragma unroll
                 for (int c = 0; c < D / 64; ++c)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        umma_bf16(tmem_base + TM_S, smem_desc(aQ + c * 16384 + k * 32, 16, 1024), smem_desc(aK + c * 16384 + k * 32, 16, 1024),
-                                  idesc_qk, (c > 0 || k > 0) ? 1u : 0u);
-                        umma_bf16(tmem_base + TM_DP, smem_desc(aDO + c * 16384 + k * 32, 16, 1024), smem_desc(aV + c * 16384 + k * 32, 16, 1024),
-                                  idesc_qk, (c > 0 || k > 0) ? 1u : 0u);
-                    }
-                umma_commit(sdp_full);
-                ok = mbar_wait(pds_ready, (uint32_t)(it & 1), P.status);
+                    for (int k = 0; k < 4; ++k)
+                        umma_bf16(tmem_base + TM_S, smem_desc(aK + c * 16384 + k * 32, 16, 1024), smem_desc(aQ + c * 16384 + k * 32, 16, 1024), idesc_t,
+                                  (c > 0 || k > 0) ? 1u : 0u);
+                umma_commit(s_full);
+                return true;
+            };
+            bool ok = mbar_wait(kv_full, 0, P.status) && issue_s(0);
+            for (int it = 0; it < n_it && ok; ++it) {
+                const uint32_t aQ = smem_u32(sq + (it & 1) * S::TILE), aDO = smem_u32(sdo + (it % NDO) * S::TILE);
+                const uint32_t ph = (uint32_t)(it & 1), acc = it > 0 ? 1u : 0u;
+                ok = mbar_wait(&do_full[it % NDO], (uint32_t)((it / NDO) & 1), P.status) && mbar_wait(p_ready, ph, P.status);
                 if (!ok) break;
                 tc_fence_after();
-                const uint32_t acc = it > 0 ? 1u : 0u;
 #pragma unroll
-                for (int kq = 0; kq < 8; ++kq) {      // K dimension = the 128 query rows, 16 per step: 2048 B further down each chunk
-                    umma_bf16(tmem_base + TM_DV, smem_desc(aP + kq * 2048, 16384, 1024), smem_desc(aDO + kq * 2048, 16384, 1024), idesc_tt,
-                              (kq > 0) ? 1u : acc);
-                    umma_bf16(tmem_base + TM_DK, smem_desc(aDS + kq * 2048, 16384, 1024), smem_desc(aQ + kq * 2048, 16384, 1024), idesc_tt,
-                              (kq > 0) ? 1u : acc);
+                for (int kq = 0; kq < 8; ++kq)        // K dimension = the 128 queries, 16 per step: 2048 B further down each chunk of dO
+                    umma_bf16_ts(tmem_base + TM_DV, tmem_base + TM_S + (uint32_t)((kq >> 2) * 64 + (kq & 3) * 8), smem_desc(aDO + kq * 2048, 16384, 1024), idesc_k,
+                                 (kq > 0) ? 1u : acc);
+                if (TM_DQ == TM_DP && it > 0) {       // dQ_i-1 leaves these columns while dV runs
+                    ok = mbar_wait(dq_read, ph ^ 1, P.status);
+                    if (!ok) break;
+                    tc_fence_after();
                 }
 #pragma unroll
-                for (int c = 0; c < 2; ++c)           // K dimension = the 128 keys: two 64-key chunks of dS, 16 keys = 32 B per step
+                for (int c = 0; c < D / 64; ++c)
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
-                        umma_bf16(tmem_base + TM_S, smem_desc(aDS + c * 16384 + k * 32, 16, 1024),
-                                  smem_desc(aK + (c * 4 + k) * 2048, 16384, 1024), idesc_dq, (c > 0 || k > 0) ? 1u : 0u);
-                umma_commit(&qdo_empty[stg]);
+                        umma_bf16(tmem_base + TM_DP, smem_desc(aV + c * 16384 + k * 32, 16, 1024), smem_desc(aDO + c * 16384 + k * 32, 16, 1024), idesc_t,
+                                  (c > 0 || k > 0) ? 1u : 0u);
+                umma_commit(dp_full);
+                umma_commit(&do_empty[it % NDO]);
+                if (it + 1 < n_it) ok = issue_s(it + 1);
+                if (ok) ok = mbar_wait(ds_ready, ph, P.status);
+                if (ok && TM_DQ != TM_DP && it > 0) ok = mbar_wait(dq_read, ph ^ 1, P.status);
+                if (!ok) break;
+                tc_fence_after();
+#pragma unroll
+                for (int kq = 0; kq < 8; ++kq)
+                    umma_bf16(tmem_base + TM_DK, smem_desc(aDS + (kq >> 2) * 16384 + (kq & 3) * 32, 16, 1024), smem_desc(aQ + kq * 2048, 16384, 1024), idesc_k,
+                              (kq > 0) ? 1u : acc);
+                umma_commit(&q_empty[it & 1]);
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)        // K dimension = the 128 keys
+                    umma_bf16(tmem_base + TM_DQ, smem_desc(aDS + kk * 2048, 16384, 1024), smem_desc(aK + kk * 2048, 16384, 1024), idesc_q, kk > 0 ? 1u : 0u);
                 umma_commit(dq_full);
             }
+            umma_commit(all_done);
             if (!ok) *abort_flag = 1;
         }
-    } else {
-        // ---------------------------------------------------------------------------- compute warps
-        const int row = 32 * (warp & 3) + lane;          // query row of the block = TMEM lane (key row in the final read-out)
-        const int hf = warp >> 2;
-        const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
+    } else if (warp >= 12) {
+        // ---------------------------------------------------------------------------- dQ warps
+        regs_inc<REGS_DQ>();
+        const int row = 32 * (warp & 3) + lane;          // query row of the block = TMEM lane
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16) + TM_DQ;
+        const bool elected = warp == 12 && lane == 0;
         bool ok = true;
+        int piece = 0;
+#pragma unroll 1
         for (int it = 0; it < n_it; ++it) {
             const int h = head0 + it / per_head, i = i_start + it % per_head;
-            const int q_idx = i * 128 + row;
-            const bool q_valid = q_idx < P.Tq;
-            const size_t stat = ((size_t)b * P.H + h) * P.Tq + q_idx;
-            const float lse2 = q_valid ? P.lse[stat] * 1.4426950408889634f : INFINITY;       // +inf: P = 0 for padded rows
-            const float dlt = q_valid ? P.delta[stat] : 0.f;
-            if (ok && !*abort_flag) ok = mbar_wait(sdp_full, (uint32_t)(it & 1), P.status);
+            if (ok && !*abort_flag) ok = mbar_wait(dq_full, (uint32_t)(it & 1), P.status);
             else ok = false;
             tc_fence_after();
-            const int kbase = key0 + hf * 64;
-            const int q_pos = q_idx + P.q_offset;
-            const bool need_mask = (kbase + 64 > P.Tk) || (P.causal && kbase + 63 > i * 128 + P.q_offset);
-            uint32_t pp[32], dd[32];
+            float r[D];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                uint32_t rs[32], rd[32];
-                tmem_ld32(lane_addr + TM_S + (uint32_t)(hf * 64 + c * 32), rs);
-                tmem_ld32(lane_addr + TM_DP + (uint32_t)(hf * 64 + c * 32), rd);
-                tmem_ld_wait();
-#pragma unroll
-                for (int e = 0; e < 32; e += 2) {
-                    float p0 = exp2f(__uint_as_float(rs[e]) * P.scale_log2 - lse2), p1 = exp2f(__uint_as_float(rs[e + 1]) * P.scale_log2 - lse2);
-                    if (need_mask) {
-                        const int k0 = kbase + c * 32 + e;
-                        if (k0 >= P.Tk || (P.causal && k0 > q_pos)) p0 = 0.f;
-                        if (k0 + 1 >= P.Tk || (P.causal && k0 + 1 > q_pos)) p1 = 0.f;
-                    }
-                    const float d0 = p0 * (__uint_as_float(rd[e]) - dlt) * P.scale, d1 = p1 * (__uint_as_float(rd[e + 1]) - dlt) * P.scale;
-                    const __nv_bfloat162 ph = __floats2bfloat162_rn(p0, p1), dh = __floats2bfloat162_rn(d0, d1);
-                    pp[c * 16 + e / 2] = *reinterpret_cast<const uint32_t*>(&ph);
-                    dd[c * 16 + e / 2] = *reinterpret_cast<const uint32_t*>(&dh);
-                }
-            }
-            {
-                uint8_t* prow = sp + hf * 16384 + row * 128;
-                uint8_t* drow = sds + hf * 16384 + row * 128;
-#pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    const int off = (c ^ (row & 7)) * 16;
-                    *reinterpret_cast<uint4*>(prow + off) = make_uint4(pp[4 * c], pp[4 * c + 1], pp[4 * c + 2], pp[4 * c + 3]);
-                    *reinterpret_cast<uint4*>(drow + off) = make_uint4(dd[4 * c], dd[4 * c + 1], dd[4 * c + 2], dd[4 * c + 3]);
-                }
-            }
-            fence_proxy_async();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(pds_ready);
-            // ---- dQ_i: read back my half of the row and add it to global memory
-            if (ok) ok = mbar_wait(dq_full, (uint32_t)(it & 1), P.status);
-            tc_fence_after();
-            float* dqp = P.dq + (((size_t)b * P.Tq + q_idx) * P.H + h) * D + hf * (D / 2);
-#pragma unroll
-            for (int c = 0; c < D / 64; ++c) {
-                uint32_t r[32];
-                tmem_ld32(lane_addr + TM_S + (uint32_t)(hf * (D / 2) + c * 32), r);
-                tmem_ld_wait();
-                if (q_valid && ok) {
-#pragma unroll
-                    for (int e = 0; e < 32; e += 4)
-                        red_add_v4(dqp + c * 32 + e, __uint_as_float(r[e]), __uint_as_float(r[e + 1]), __uint_as_float(r[e + 2]), __uint_as_float(r[e + 3]));
-                }
-            }
+            for (int c = 0; c < D / 32; ++c) tmem_ld32(lane_addr + (uint32_t)(c * 32), reinterpret_cast<uint32_t*>(r) + c * 32);
+            tmem_ld_wait();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(dq_read);
-        }
-        // ---- dK_j, dV_j: lanes are key rows now
-        const int key = key0 + row;
-        if (n_it > 0 && ok && !*abort_flag) {
-            tc_fence_after();
 #pragma unroll
+            for (int c = 0; c < D / 32; ++c, ++piece) {
+                uint8_t* buf = stg + (piece & 1) * S::STG;
+                if (elected) bulk_wait_read<1>();        // the piece before last has left this buffer
+                dq_sync();
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    *reinterpret_cast<float4*>(buf + row * 128 + ((u ^ (row & 7)) * 16)) =
+                        make_float4(r[c * 32 + 4 * u], r[c * 32 + 4 * u + 1], r[c * 32 + 4 * u + 2], r[c * 32 + 4 * u + 3]);
+                fence_proxy_async();
+                dq_sync();
+                if (elected) {
+                    if (ok) tma_reduce_add_3d(&tmDQ, buf, h * D + c * 32, i * 128, b);
+                    bulk_commit();
+                }
+            }
+        }
+        if (elected) bulk_wait<0>();
+        if (!ok) *abort_flag = 1;
+    } else {
+        // ---------------------------------------------------------------------------- compute warps
+        regs_inc<REGS_COMPUTE>();
+        const int row = 32 * (warp & 3) + lane;          // key of the block = TMEM lane
+        const int hf = warp >> 2;                        // which 64 queries
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(32 * (warp & 3)) << 16);
+        const int key = key0 + row;
+        bool ok = true;
+        // thread x brings lse (x < 128) or delta of query x % 128 of a block, ready to use: lse in powers of two, delta times the scale
+        auto row_value = [&](int it) {
+            const int h = head0 + it / per_head, q = (i_start + it % per_head) * 128 + (threadIdx.x & 127);
+            const bool is_lse = threadIdx.x < 128;
+            if (q >= P.Tq) return is_lse ? INFINITY : 0.f;                  // P = 0 for rows past the end
+            const size_t at = ((size_t)b * P.H + h) * P.Tq + q;
+            return is_lse ? P.lse[at] * 1.4426950408889634f : P.delta[at] * P.scale;
+        };
+        if (n_it > 0) {
+            srow[threadIdx.x] = row_value(0);
+            compute_sync();
+        }
+#pragma unroll 1
+        for (int it = 0; it < n_it; ++it) {
+            const int q0 = (i_start + it % per_head) * 128;
+            const float next_row = it + 1 < n_it ? row_value(it + 1) : 0.f;
+            const float4* lse4 = reinterpret_cast<const float4*>(srow + (it & 1) * 256 + hf * 64);
+            const float4* dlt4 = lse4 + 32;
+            if (ok && !*abort_flag) ok = mbar_wait(s_full, (uint32_t)(it & 1), P.status);
+            else ok = false;
+            tc_fence_after();
+            float p[64];
+            tmem_ld32(lane_addr + TM_S + (uint32_t)(hf * 64), reinterpret_cast<uint32_t*>(p));
+            tmem_ld32(lane_addr + TM_S + (uint32_t)(hf * 64 + 32), reinterpret_cast<uint32_t*>(p) + 32);
+            tmem_ld_wait();
+#pragma unroll
+            for (int e = 0; e < 16; ++e) {
+                const float4 l = lse4[e];
+                p[4 * e] = exp2f(p[4 * e] * P.scale_log2 - l.x);
+                p[4 * e + 1] = exp2f(p[4 * e + 1] * P.scale_log2 - l.y);
+                p[4 * e + 2] = exp2f(p[4 * e + 2] * P.scale_log2 - l.z);
+                p[4 * e + 3] = exp2f(p[4 * e + 3] * P.scale_log2 - l.w);
+            }
+            const int qf = q0 + hf * 64;
+            const bool need_mask = (key0 + 128 > P.Tk) || (P.causal && key0 + 127 > qf + P.q_offset);
+            const int first = key >= P.Tk ? 64 : P.causal ? key - P.q_offset - qf : 0;        // of this thread's queries, those from here on see the key
+            if (need_mask) {
+#pragma unroll
+                for (int e = 0; e < 64; ++e)
+                    if (e < first) p[e] = 0.f;
+            }
+            {
+                uint32_t pk[32];
+#pragma unroll
+                for (int e = 0; e < 32; ++e) {
+                    const __nv_bfloat162 h2 = __floats2bfloat162_rn(p[2 * e], p[2 * e + 1]);
+                    pk[e] = *reinterpret_cast<const uint32_t*>(&h2);
+                }
+                tmem_st32(lane_addr + TM_S + (uint32_t)(hf * 64), pk);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(p_ready);
+            if (ok && !*abort_flag) ok = mbar_wait(dp_full, (uint32_t)(it & 1), P.status);
+            else ok = false;
+            tc_fence_after();
+            uint8_t* drow = sds + hf * 16384 + row * 128;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float d[32];
+                tmem_ld32(lane_addr + TM_DP + (uint32_t)(hf * 64 + c * 32), reinterpret_cast<uint32_t*>(d));
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float4 dl = dlt4[c * 8 + e];
+                    d[4 * e] = p[c * 32 + 4 * e] * (d[4 * e] * P.scale - dl.x);
+                    d[4 * e + 1] = p[c * 32 + 4 * e + 1] * (d[4 * e + 1] * P.scale - dl.y);
+                    d[4 * e + 2] = p[c * 32 + 4 * e + 2] * (d[4 * e + 2] * P.scale - dl.z);
+                    d[4 * e + 3] = p[c * 32 + 4 * e + 3] * (d[4 * e + 3] * P.scale - dl.w);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    uint4 o;
+                    __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) oh[x] = __floats2bfloat162_rn(d[8 * u + 2 * x], d[8 * u + 2 * x + 1]);
+                    *reinterpret_cast<uint4*>(drow + (((c * 4 + u) ^ (row & 7)) * 16)) = o;
+                }
+            }
+            srow[((it + 1) & 1) * 256 + threadIdx.x] = next_row;
+            fence_proxy_async();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(ds_ready);
+            compute_sync();                   // the next block's lse and delta are there
+        }
+        // ---- dK_j, dV_j
+        if (n_it > 0) {
+            if (ok && !*abort_flag) ok = mbar_wait(all_done, 0, P.status);
+            else ok = false;
+            tc_fence_after();
+#pragma unroll 1
             for (int which = 0; which < 2; ++which) {
                 __nv_bfloat16* outp = (which ? P.dk : P.dv) + (size_t)part * P.B * P.Tk * P.Hk * D + (((size_t)b * P.Tk + key) * P.Hk + hk) * D +
                                       hf * (D / 2);
@@ -625,7 +734,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     uint32_t r[32];
                     tmem_ld32(lane_addr + (which ? TM_DK : TM_DV) + (uint32_t)(hf * (D / 2) + c * 32), r);
                     tmem_ld_wait();
-                    if (key < P.Tk) {
+                    if (key < P.Tk && ok) {
 #pragma unroll
                         for (int e = 0; e < 32; e += 8) {
                             uint4 o;
@@ -637,7 +746,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                     }
                 }
             }
-        } else if (n_it == 0 && key < P.Tk) {
+        } else if (key < P.Tk) {
             // no query block sees these keys: their gradients are zero
             const size_t base = (size_t)part * P.B * P.Tk * P.Hk * D + (((size_t)b * P.Tk + key) * P.Hk + hk) * D;
             for (int d = hf * (D / 2); d < (hf + 1) * (D / 2); ++d) {
@@ -656,7 +765,8 @@ template <int D>
 static int launch_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* delta, float* dq, void* dk,
                       void* dv, int B, int Tq, int Tk, int H, int Hk, int causal, float scale, int q_offset, int gsplit, int* status,
                       cudaStream_t st) {
-    CUtensorMap mq, mk, mv, mdo;
+    CUtensorMap mq, mk, mv, mdo, mdq;
+    if (ptb_make_tmap_f32_3d(&mdq, dq, (long long)H * D, Tq, B, 32, 128)) return -1;
     if (ptb_make_tmap_bf16(&mq, q, (long long)H * D, (long long)B * Tq, (long long)H * D, 64, 128)) return -1;
     if (ptb_make_tmap_bf16(&mdo, dout, (long long)H * D, (long long)B * Tq, (long long)H * D, 64, 128)) return -1;
     if (ptb_make_tmap_bf16(&mk, k, (long long)Hk * D, (long long)B * Tk, (long long)Hk * D, 64, 128)) return -1;
@@ -667,11 +777,11 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
         attr = true;
     }
     BwdParams p;
-    p.lse = lse; p.delta = delta; p.dq = dq; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
+    p.lse = lse; p.delta = delta; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
     p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
     p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status; p.gsplit = gsplit;
     dim3 grid((Tk + 127) / 128, Hk * gsplit, B);
-    bwd_kernel<D><<<grid, NTHREADS, SmB<D>::TOTAL, st>>>(mq, mk, mv, mdo, p);
+    bwd_kernel<D><<<grid, BWD_THREADS, SmB<D>::TOTAL, st>>>(mq, mk, mv, mdo, mdq, p);
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }

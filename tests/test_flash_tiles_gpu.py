@@ -56,3 +56,19 @@ def test_packed_sequences(lens, H, Hk, D, packed):
             continue
         want = attention_reference(q[None, a:b].double(), k[None, a:b].double(), v[None, a:b].double(), True)[0][0]
         assert _rel(o[a:b], want) < 4e-3, i
+
+
+@pytest.mark.parametrize("B,Tq,Tk,H,Hk,D,causal,off", SHAPES)
+def test_backward_tiles(B, Tq, Tk, H, Hk, D, causal, off):
+    from prometorch_b200.ops.attention import attention_reference, flash_attention
+    g = torch.Generator(device="cuda").manual_seed(Tq * Tk)
+    q, k, v = (torch.randn(B, t, h, D, device="cuda", generator=g).bfloat16().requires_grad_() for t, h in ((Tq, H), (Tk, Hk), (Tk, Hk)))
+    do = torch.randn(B, Tq, H, D, device="cuda", generator=g).bfloat16()
+    r = [t.detach().double().requires_grad_() for t in (q, k, v)]
+    skip = max(0, -off) if causal else 0          # rows that see no key: no gradient
+    ro = attention_reference(r[0][:, skip:], r[1], r[2], causal, off + skip)[0]
+    got = torch.autograd.grad(flash_attention(q, k, v, causal=causal, q_offset=off), (q, k, v), do)
+    want = torch.autograd.grad(ro, r, do[:, skip:].double())
+    for a, b in zip(got, want):
+        # P, dS and the results rounded to bf16 once each, delta from an output rounded to bf16; a single key has no gradient but rounding
+        assert float((a.double() - b).norm()) < 6e-3 * float(b.norm()) + 2 ** -9 * float(do.norm())
