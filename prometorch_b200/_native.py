@@ -89,6 +89,10 @@ def _declare(L: C.CDLL):
     L.ptb_engine_kv_cache.restype = ci
     L.ptb_dequant_weight.argtypes = [vp, ci, ci, ci, ci, vp, vp]
     L.ptb_dequant_weight.restype = ci
+    L.ptb_dequant_weights.argtypes = [vp, vp, vp, ci, ci, ci, vp, vp]
+    L.ptb_dequant_weights.restype = ci
+    L.ptb_prompt_heads.argtypes = [vp, ci, ci, ci, ci, vp, vp, ci, C.c_float, vp, vp, ci, ci, vp, vp, ci, vp]
+    L.ptb_prompt_heads.restype = ci
     L.ptb_dequant_rows.argtypes = [vp, ci, ci, ci, vp, ci, cf, ci, vp, vp, vp]
     L.ptb_dequant_rows.restype = ci
 

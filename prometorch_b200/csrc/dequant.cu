@@ -44,18 +44,33 @@ __device__ __forceinline__ uint4 pack8(const float* v) {
 // pieces of the bf16 rows, all loads of the eight rows before the first store.  Bound by the bytes written (2 a value against 0.56 or
 // 0.82 read); one value a thread, with its scales unpacked again for each, took 35 us on average over the matrices of a 2560-wide layer
 // (a prompt of 1999 tokens through 12 such layers: 15.1 ms, now 13.0).
-constexpr int DQ_WARPS = 8;
-template <int QT>
-__global__ void __launch_bounds__(DQ_WARPS * 32) dequant_t16_vec_kernel(const uint8_t* __restrict__ w, int N, int nblk, __nv_bfloat16* __restrict__ out) {
+// Matrices of one width that are read together (q, k, v; gate, up) are one launch into one stack of rows, each with its own type.
+constexpr int DQ_WARPS = 8, DQ_PARTS = 4;
+struct DequantGroup {
+    const uint8_t* w[DQ_PARTS];
+    int qtype[DQ_PARTS], rows[DQ_PARTS], row0[DQ_PARTS];
+    long long first[DQ_PARTS + 1];      // first item of each part, the unused ones and the end last
+    int nblk;
+    __nv_bfloat16* out;
+};
+__global__ void __launch_bounds__(DQ_WARPS * 32) dequant_t16_vec_kernel(const __grid_constant__ DequantGroup G) {
     const int lane = threadIdx.x & 31;
-    const long long item = (long long)blockIdx.x * DQ_WARPS + (threadIdx.x >> 5);       // (tile, block, upper or lower eight rows)
+    long long item = (long long)blockIdx.x * DQ_WARPS + (threadIdx.x >> 5);       // (part, tile, block, upper or lower eight rows)
+    if (item >= G.first[DQ_PARTS]) return;
+    int part_no = 0;
+#pragma unroll
+    for (int i = 1; i < DQ_PARTS; ++i) part_no += item >= G.first[i];
+    item -= G.first[part_no];
+    const uint8_t* __restrict__ w = G.w[part_no];
+    const int N = G.rows[part_no], nblk = G.nblk;
+    __nv_bfloat16* __restrict__ out = G.out + (size_t)G.row0[part_no] * nblk * 256;
     const int r8 = (int)(item & 1) * 8;
     const int b = (int)((item >> 1) % nblk), tile = (int)((item >> 1) / nblk);
     const int row0 = tile * 16 + r8;
     if (row0 >= N) return;
     __nv_bfloat16* o = out + (size_t)row0 * nblk * 256 + (size_t)b * 256;
     const size_t pitch = (size_t)nblk * 256;
-    if constexpr (QT == QT_Q4K) {
+    if (G.qtype[part_no] == QT_Q4K) {
         const uint8_t* blk = w + (((size_t)tile * nblk + b) * 16 + r8) * 144;
         const int rr = lane >> 4, g = (lane >> 2) & 3, part = lane & 3;                 // 64-value group, its eight bytes
         uint4 head[4];
@@ -214,9 +229,78 @@ __global__ void __launch_bounds__(256) dequant_rows_kernel(const uint8_t* __rest
     out[(size_t)t * nblk * 256 + i] = __float2bfloat16_rn(v * scale);
 }
 
+// D / 4 lanes a head, four values a lane: two neighbours of each half.  Bound by bytes (each value read once, k and v written twice); as
+// norms, rotations, conversions and copies of their own these were eight passes and eight launches a layer.
+template <int D>
+__global__ void __launch_bounds__(256) prompt_heads_kernel(__nv_bfloat16* __restrict__ qkv, long long heads, int H, int Hk, const float* __restrict__ q_norm,
+                                                           const float* __restrict__ k_norm, float more, float eps, const float* __restrict__ cos,
+                                                           const float* __restrict__ sin, int neox, int pos0, __half* __restrict__ kc, __half* __restrict__ vc, int S) {
+    constexpr int LANES = D / 4;
+    const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) / LANES;
+    const int l = threadIdx.x % LANES, per = H + 2 * Hk;
+    const bool on = at < heads;
+    const int t = on ? (int)(at / per) : 0, h = on ? (int)(at % per) : 0;
+    __nv_bfloat162* row = reinterpret_cast<__nv_bfloat162*>(qkv + (on ? at : 0) * D);
+    const __nv_bfloat162 ra = row[l], rb = row[D / 4 + l];
+    float2 a = __bfloat1622float2(ra), b = __bfloat1622float2(rb);
+    const float* w = h < H ? q_norm : h < H + Hk ? k_norm : nullptr;
+    float ss = a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y;
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (!on) return;
+    if (h < H + Hk) {
+        if (w) {
+            const float rs = rsqrtf(ss / (float)D + eps);
+            const float2 wa = *reinterpret_cast<const float2*>(w + 2 * l), wb = *reinterpret_cast<const float2*>(w + D / 2 + 2 * l);
+            a.x *= rs * (wa.x + more); a.y *= rs * (wa.y + more); b.x *= rs * (wb.x + more); b.y *= rs * (wb.y + more);
+        }
+        const float* cs = cos + (size_t)(pos0 + t) * (D / 2);
+        const float* sn = sin + (size_t)(pos0 + t) * (D / 2);
+        if (neox) {
+            const float2 c = *reinterpret_cast<const float2*>(cs + 2 * l), s = *reinterpret_cast<const float2*>(sn + 2 * l);
+            const float2 x = a;
+            a.x = x.x * c.x - b.x * s.x; b.x = b.x * c.x + x.x * s.x;
+            a.y = x.y * c.y - b.y * s.y; b.y = b.y * c.y + x.y * s.y;
+        } else {
+            const float c0 = cs[l], s0 = sn[l], c1 = cs[D / 4 + l], s1 = sn[D / 4 + l];
+            a = make_float2(a.x * c0 - a.y * s0, a.y * c0 + a.x * s0);
+            b = make_float2(b.x * c1 - b.y * s1, b.y * c1 + b.x * s1);
+        }
+        row[l] = __floats2bfloat162_rn(a.x, a.y);
+        row[D / 4 + l] = __floats2bfloat162_rn(b.x, b.y);
+    }
+    if (h >= H) {
+        const bool is_k = h < H + Hk;
+        __half2* dst = reinterpret_cast<__half2*>((is_k ? kc : vc) + ((size_t)(is_k ? h - H : h - H - Hk) * S + pos0 + t) * D);
+        dst[l] = __floats2half2_rn(a.x, a.y);
+        dst[D / 4 + l] = __floats2half2_rn(b.x, b.y);
+    }
+}
+
 }  // namespace ptb
 
 using namespace ptb;
+
+static int dequant_group(const void* const* w, const int* qtypes, const int* rows, int n, int nblk, void* out, cudaStream_t st) {
+    DequantGroup g;
+    memset(&g, 0, sizeof(g));
+    g.nblk = nblk;
+    g.out = (__nv_bfloat16*)out;
+    long long items = 0;
+    int row = 0;
+    for (int i = 0; i < DQ_PARTS; ++i) {
+        g.first[i] = items;
+        if (i >= n) continue;
+        g.w[i] = (const uint8_t*)w[i]; g.qtype[i] = qtypes[i]; g.rows[i] = rows[i]; g.row0[i] = row;
+        items += (long long)((rows[i] + 15) / 16) * 2 * nblk;
+        row += rows[i];
+    }
+    for (int i = n; i < DQ_PARTS; ++i) g.first[i] = items;
+    g.first[DQ_PARTS] = items;
+    dequant_t16_vec_kernel<<<(unsigned)((items + DQ_WARPS - 1) / DQ_WARPS), DQ_WARPS * 32, 0, st>>>(g);
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
 
 // w: a matrix of N rows x cols in a GEMV streaming layout -> out bf16 [N, cols] row-major.
 // layout: 0 = [segment][row][segment bytes], 1 = tiles of 16 rows.
@@ -228,14 +312,7 @@ PTB_API int ptb_dequant_weight(const void* w, int qtype, int layout, int N, int 
         return -1;
     }
     const int nblk = cols / 256;
-    if (layout == 1 && !tile_only && !(((uintptr_t)w | (uintptr_t)out) & 15)) {
-        const long long items = (long long)((N + 15) / 16) * 2 * nblk;
-        const unsigned grid = (unsigned)((items + DQ_WARPS - 1) / DQ_WARPS);
-        if (qtype == QT_Q4K) dequant_t16_vec_kernel<QT_Q4K><<<grid, DQ_WARPS * 32, 0, st>>>((const uint8_t*)w, N, nblk, (__nv_bfloat16*)out);
-        else dequant_t16_vec_kernel<QT_Q6K><<<grid, DQ_WARPS * 32, 0, st>>>((const uint8_t*)w, N, nblk, (__nv_bfloat16*)out);
-        PTB_CUDA_OK(cudaGetLastError());
-        return 0;
-    }
+    if (layout == 1 && !tile_only && !(((uintptr_t)w | (uintptr_t)out) & 15)) return dequant_group(&w, &qtype, &N, 1, nblk, out, st);
     if (layout == 1) {
         dequant_t16_kernel<<<dim3(nblk, (N + 3) / 4), 256, 0, st>>>((const uint8_t*)w, qtype, N, nblk, (__nv_bfloat16*)out);
         PTB_CUDA_OK(cudaGetLastError());
@@ -244,6 +321,40 @@ PTB_API int ptb_dequant_weight(const void* w, int qtype, int layout, int N, int 
     const int KS = (nblk + GEMV_SEG_BLOCKS - 1) / GEMV_SEG_BLOCKS;
     dequant_segmajor_kernel<<<dim3(nblk, (N + 3) / 4), 256, 0, st>>>((const uint8_t*)w, qtype, N, nblk, KS, nblk / KS, nblk % KS,
                                                                     (__nv_bfloat16*)out);
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+// `n` matrices of the same width, one below the other in `out` [sum of rows, cols]: one launch where they are Q4_K or Q6_K in tiles of 16 rows.
+PTB_API int ptb_dequant_weights(const void* const* w, const int* qtypes, const int* rows, int n, int layout, int cols, void* out, cudaStream_t st) {
+    if (n < 1 || n > DQ_PARTS || cols % 256) { ptb_set_error("dequant: %d matrices of %d columns not supported", n, cols); return -1; }
+    bool one = layout == 1 && !((uintptr_t)out & 15);
+    for (int i = 0; i < n; ++i) one = one && rows[i] > 0 && (qtypes[i] == QT_Q4K || qtypes[i] == QT_Q6K) && !((uintptr_t)w[i] & 15);
+    if (one) return dequant_group(w, qtypes, rows, n, cols / 256, out, st);
+    __nv_bfloat16* o = (__nv_bfloat16*)out;
+    for (int i = 0; i < n; ++i) {
+        if (ptb_dequant_weight(w[i], qtypes[i], layout, rows[i], cols, o, st)) return -1;
+        o += (size_t)rows[i] * cols;
+    }
+    return 0;
+}
+
+// What stands between the packed projection of a prompt and its attention: norm of the q and k heads (weights fp32 [D] or null; add_one: they are
+// stored less one), rotary positions from pos0 (pairs (j, j + D/2), or (2j, 2j + 1)), both in place and rounded once, and k and v into the
+// fp16 cache [Hk, S, D].  qkv bf16 [T, (H + 2 Hk) D]; cos, sin fp32 [S, D/2]; D 64 or 128.
+PTB_API int ptb_prompt_heads(void* qkv, int T, int H, int Hk, int D, const float* q_norm, const float* k_norm, int add_one, float eps, const float* cos,
+                             const float* sin, int neox, int pos0, void* k_cache, void* v_cache, int S, cudaStream_t st) {
+    if (T <= 0) return 0;
+    if (pos0 < 0 || pos0 + T > S) { ptb_set_error("prompt heads: positions %d .. %d outside a cache of %d", pos0, pos0 + T, S); return -1; }
+    if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos | (uintptr_t)sin) & 7) { ptb_set_error("prompt heads: needs 8-byte aligned buffers"); return -1; }
+    const long long heads = (long long)T * (H + 2 * Hk);
+    auto go = [&](auto kern, int per_cta) {
+        kern<<<(unsigned)((heads + per_cta - 1) / per_cta), 256, 0, st>>>((__nv_bfloat16*)qkv, heads, H, Hk, q_norm, k_norm, add_one ? 1.f : 0.f, eps, cos, sin, neox, pos0,
+                                                                        (__half*)k_cache, (__half*)v_cache, S);
+    };
+    if (D == 128) go(prompt_heads_kernel<128>, 8);
+    else if (D == 64) go(prompt_heads_kernel<64>, 16);
+    else { ptb_set_error("prompt heads: head size %d not in {64, 128}", D); return -1; }
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }

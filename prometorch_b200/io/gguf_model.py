@@ -474,14 +474,15 @@ class GGUFModel:
         under tensor parallelism, on every rank over its own heads and FFN columns with two all-reduces per layer."""
         return not self.cfg.swa_window and self.cfg.head_dim in (64, 128)
 
-    def _dequant(self, pw: "PackedWeight") -> torch.Tensor:
-        """bf16 ``[rows, cols]`` copy of a packed matrix in a scratch buffer shared by all matrices of that shape."""
-        key = (pw.rows, pw.cols)
-        buf = self._dq_scratch.get(key)
+    def _dequant(self, *pws: "PackedWeight") -> torch.Tensor:
+        """bf16 ``[rows, cols]`` copy of packed matrices of one width, one below the other, in a scratch buffer shared by all of that shape."""
+        n, rows, cols = len(pws), sum(pw.rows for pw in pws), pws[0].cols
+        buf = self._dq_scratch.get((rows, cols))
         if buf is None:
-            buf = self._dq_scratch[key] = torch.empty(pw.rows, pw.cols, dtype=torch.bfloat16, device=self.device)
+            buf = self._dq_scratch[rows, cols] = torch.empty(rows, cols, dtype=torch.bfloat16, device=self.device)
         st = torch.cuda.current_stream(self.device).cuda_stream
-        N.check(self._lib.ptb_dequant_weight(pw.data.data_ptr(), pw.qtype, pw.layout, pw.rows, pw.cols, buf.data_ptr(), st), "dequant")
+        N.check(self._lib.ptb_dequant_weights((C.c_void_p * n)(*[pw.data.data_ptr() for pw in pws]), (C.c_int * n)(*[pw.qtype for pw in pws]),
+                                              (C.c_int * n)(*[pw.rows for pw in pws]), n, pws[0].layout, cols, buf.data_ptr(), st), "dequant")
         return buf
 
     def _kv_views(self, layer: int):
@@ -494,8 +495,8 @@ class GGUFModel:
     @torch.no_grad()
     def prefill(self, tokens: Sequence[int], pos0: int = 0, return_logits: bool = False):
         """Run ``tokens`` at positions ``pos0 ..`` through the model in ONE batched pass that fills the KV cache:
-        weights are dequantised to bf16 layer by layer and every projection is a tcgen05 GEMM over all prompt
-        tokens, attention is the FlashAttention kernel.  Nothing is returned; decoding continues with
+        weights are dequantised to bf16 layer by layer (those with one input into one matrix) and every projection is a tcgen05 GEMM
+        over all prompt tokens, attention is the FlashAttention kernel.  Nothing is returned; decoding continues with
         ``forward_decode(next_token, pos0 + len(tokens))``.  (Token-by-token prefill costs one decode step each.)
         Under tensor parallelism the call is collective: every rank runs it with the same tokens.
         ``return_logits=True`` also applies the output norm and the lm_head to every position and returns fp32 logits
@@ -503,8 +504,8 @@ class GGUFModel:
         if not self.supports_prefill:
             raise NotImplementedError("batched prefill: no sliding window, head size 64 or 128")
         from ..ops import fused_ops as K
-        from ..ops.attention import flash_attention
-        from ..ops.gemm import linear
+        from ..ops.attention import flash_attention, flash_attention_varlen
+        from ..ops.gemm import linear, linear_add_rms_norm, linear_swiglu
         cfg, dev = self.cfg, self.device
         T = len(tokens)
         if T == 0:
@@ -531,56 +532,55 @@ class GGUFModel:
                 L[key] = None if w is None else ((w + 1.0) if cfg.gemma_norm_add_one else w).to(bf)
             return L[key]
 
-        def proj(h, pw):
-            y = linear(h, self._dequant(pw), None)
-            return y if pw.bias is None else y + pw.bias.to(bf)
+        def bias_of(L, name, parts):      # of stacked matrices, fp32; None if none has one
+            if name not in L:
+                some = any(L[n].bias is not None for n in parts)
+                L[name] = torch.cat([torch.zeros(L[n].rows, device=dev) if L[n].bias is None else L[n].bias.float() for n in parts]) if some else None
+            return L[name]
 
-        def ksplit(h, pw):
-            """A projection split along K over the ranks (attention output, FFN down): every rank multiplies its own
-            columns and the partial results are summed in fp32 across the ranks (collective: all ranks prefill together)."""
-            y = proj(h, pw)
+        def ksplit_norm(h, pw, L, post, norm):
+            """A projection into the residual stream, split along K over the ranks (every rank multiplies its own columns and the partial
+            results are summed in fp32 across the ranks; collective: all ranks prefill together), and the norm that follows:
+            the normed rows and the new stream."""
+            w = self._dequant(pw)
+            if self.tp_world == 1 and pw.bias is None and L[post] is None and norm is not None:
+                return linear_add_rms_norm(h, w, x, norm, eps)
+            y = linear(h, w, pw.bias)
             if self.tp_world > 1:
                 y32 = y.float()
                 self.symm.dist.all_reduce(y32, group=self.symm.pg)
                 y = y32.to(bf)
-            return y
+            if L[post] is not None:
+                y = K.rms_norm(y, nw(L, post), eps)
+            return K.add_rms_norm(y, x, norm, eps) if norm is not None else (None, x + y)
 
+        if return_logits and not hasattr(self, "_out_norm_bf16"):
+            w = self.out_norm
+            self._out_norm_bf16 = ((w + 1.0) if cfg.gemma_norm_add_one else w).to(bf)
+        offs = [0, T]
+        offs_dev = torch.tensor(offs, dtype=torch.int32, device=dev)
+        h = K.rms_norm(x, nw(self.layers[0], "attn_norm"), eps)
         for i, L in enumerate(self.layers):
-            h = K.rms_norm(x, nw(L, "attn_norm"), eps)
-            q = proj(h, L["q"]).view(T, hq, d)
-            k = proj(h, L["k"]).view(T, hkv, d)
-            v = proj(h, L["v"]).view(T, hkv, d)
-            if L["q_norm"] is not None:
-                q = K.rms_norm(q.reshape(-1, d), nw(L, "q_norm"), eps).view(T, hq, d)
-                k = K.rms_norm(k.reshape(-1, d), nw(L, "k_norm"), eps).view(T, hkv, d)
-            q = K.rope(q.unsqueeze(0), self.cos, self.sin, bool(cfg.rope_neox), pos0)
-            k = K.rope(k.unsqueeze(0), self.cos, self.sin, bool(cfg.rope_neox), pos0)
+            last = i + 1 == len(self.layers)
+            qkv = linear(h, self._dequant(L["q"], L["k"], L["v"]), bias_of(L, "qkv_bias", ("q", "k", "v")))
             kc, vc = self._kv_views(i)
-            kc[:, pos0:pos0 + T] = k[0].permute(1, 0, 2).to(torch.float16)
-            vc[:, pos0:pos0 + T] = v.permute(1, 0, 2).to(torch.float16)
+            N.check(self._lib.ptb_prompt_heads(qkv.data_ptr(), T, hq, hkv, d, N.ptr(L["q_norm"]), N.ptr(L["k_norm"]), int(bool(cfg.gemma_norm_add_one)), eps,
+                                               self.cos.data_ptr(), self.sin.data_ptr(), int(bool(cfg.rope_neox)), pos0, kc.data_ptr(), vc.data_ptr(),
+                                               self.max_seq, st), "prompt_heads")
+            if last and not return_logits:
+                break                 # the cache is complete, and nothing reads the last layer's output
+            heads = qkv.view(T, hq + 2 * hkv, d)
             if pos0 > 0:          # earlier positions come from the cache
                 k_all = kc[:, :pos0 + T].permute(1, 0, 2).to(bf).unsqueeze(0).contiguous()
                 v_all = vc[:, :pos0 + T].permute(1, 0, 2).to(bf).unsqueeze(0).contiguous()
+                att = flash_attention(heads[None, :, :hq], k_all, v_all, causal=True, q_offset=pos0)
             else:
-                k_all, v_all = k, v.unsqueeze(0)
-            att = flash_attention(q, k_all, v_all, causal=True, q_offset=pos0).reshape(T, hq * d)
-            o = ksplit(att, L["o"])
-            if L["post_attn_norm"] is not None:
-                o = K.rms_norm(o, nw(L, "post_attn_norm"), eps)
-            x = x + o
-            h = K.rms_norm(x, nw(L, "ffn_norm"), eps)
-            g, u = proj(h, L["gate"]), proj(h, L["up"]).clone()       # gate and up share a scratch shape: keep one
-            act = torch.nn.functional.gelu(g.float(), approximate="tanh") if cfg.ffn_gelu else torch.nn.functional.silu(g.float())
-            dn = ksplit((act * u.float()).to(bf), L["down"])
-            if L["post_ffn_norm"] is not None:
-                dn = K.rms_norm(dn, nw(L, "post_ffn_norm"), eps)
-            x = x + dn
-        logits = None
-        if return_logits:
-            if not hasattr(self, "_out_norm_bf16"):
-                w = self.out_norm
-                self._out_norm_bf16 = ((w + 1.0) if cfg.gemma_norm_add_one else w).to(bf)
-            logits = linear(K.rms_norm(x, self._out_norm_bf16, eps), self._dequant(self.lm_head), None).float()
+                att = flash_attention_varlen(heads[:, :hq], heads[:, hq:hq + hkv], heads[:, hq + hkv:], offs, offs_dev)
+            h, x = ksplit_norm(att.reshape(T, hq * d), L["o"], L, "post_attn_norm", nw(L, "ffn_norm"))
+            w, gu_bias = self._dequant(L["gate"], L["up"]), bias_of(L, "gate_up_bias", ("gate", "up"))
+            act = linear_swiglu(h, w, bool(cfg.ffn_gelu)) if gu_bias is None else K.swiglu(linear(h, w, gu_bias), bool(cfg.ffn_gelu))
+            h, x = ksplit_norm(act, L["down"], L, "post_ffn_norm", self._out_norm_bf16 if last else nw(self.layers[i + 1], "attn_norm"))
+        logits = linear(h, self._dequant(self.lm_head), None).float() if return_logits else None
         torch.cuda.current_stream(dev).synchronize()
         if int(self._pf_status):
             self._pf_status.zero_()

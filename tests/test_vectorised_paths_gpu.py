@@ -64,3 +64,62 @@ def test_cross_entropy_gradient_of_the_mean(V, rows, dtype, up):
     # up to two roundings of the stored type, and the fast exponential's error (2^-21 of the largest logit)
     eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -19
     assert float((x.grad.double() - r.grad).abs().max()) <= 2 * eps * abs(up) / max(1, int((t >= 0).sum()))
+
+
+@pytest.mark.parametrize("kinds", [("Q4_K", "Q4_K", "Q6_K"), ("Q6_K", "Q4_K"), ("Q4_K", "Q8_0", "Q6_K"), ("Q6_K",)])
+@pytest.mark.parametrize("rows", [(40, 8, 24), (16, 1, 7)])
+@pytest.mark.parametrize("layout", [0, 1])
+def test_dequant_stacked(kinds, rows, layout):
+    """Several matrices into one stack: the same rows as one by one, whatever their types, also when a type has no wide form."""
+    from prometorch_b200 import _native as N
+    from prometorch_b200.io import gguf_quant as Q
+    from prometorch_b200.io.gguf_model import pack_weight
+    import ctypes as C
+    if layout == 0 and "Q8_0" in kinds:
+        pytest.skip("Q8_0 is streamed in tiles only")
+    cols, st = 768, torch.cuda.current_stream().cuda_stream
+    g = torch.Generator(device="cuda").manual_seed(sum(rows))
+    pws = [pack_weight(Q.quantize(torch.randn(r, cols, device="cuda", generator=g), Q.GGMLType[k]), Q.GGMLType[k], cols, "cuda", layout=layout)
+           for r, k in zip(rows, kinds)]
+    n, total = len(pws), sum(pw.rows for pw in pws)
+    out = torch.full((total + 1, cols), 7.0, dtype=torch.bfloat16, device="cuda")
+    N.check(N.lib().ptb_dequant_weights((C.c_void_p * n)(*[p.data.data_ptr() for p in pws]), (C.c_int * n)(*[p.qtype for p in pws]),
+                                        (C.c_int * n)(*[p.rows for p in pws]), n, layout, cols, out.data_ptr(), st), "dequant")
+    at = 0
+    for p in pws:
+        one = torch.empty(p.rows, cols, dtype=torch.bfloat16, device="cuda")
+        N.check(N.lib().ptb_dequant_weight(p.data.data_ptr(), p.qtype, layout, p.rows, cols, one.data_ptr(), st), "dequant")
+        assert torch.equal(out[at:at + p.rows], one)
+        at += p.rows
+    assert bool((out[total] == 7).all())
+
+
+@pytest.mark.parametrize("T,H,Hk,D,pos0", [(1, 1, 1, 64, 0), (7, 3, 1, 64, 5), (33, 4, 2, 128, 0), (5, 2, 2, 128, 59)])
+@pytest.mark.parametrize("neox", [True, False])
+@pytest.mark.parametrize("norm,add_one", [(True, False), (True, True), (False, False)])
+def test_prompt_heads(T, H, Hk, D, pos0, neox, norm, add_one):
+    from prometorch_b200 import _native as N
+    from prometorch_b200.ops import fused_ops as K
+    from prometorch_b200.ops.paged import rope_tables
+    S, per = 64, H + 2 * Hk
+    g = torch.Generator(device="cuda").manual_seed(T * D)
+    x = torch.randn(T, per, D, device="cuda", generator=g).bfloat16()
+    w = [torch.randn(D, device="cuda", generator=g) * 0.1 + (0 if add_one else 1) if norm else None for _ in range(2)]
+    cos, sin = rope_tables(S, D, 10000.0, "cuda")
+    kc, vc = (torch.zeros(Hk, S, D, dtype=torch.float16, device="cuda") for _ in range(2))
+    want = x.double()
+    if norm:
+        r = want * torch.rsqrt(want.square().mean(-1, keepdim=True) + 1e-6)
+        want = torch.cat([r[:, :H] * (w[0].double() + add_one), r[:, H:H + Hk] * (w[1].double() + add_one), want[:, H + Hk:]], 1)
+    qk = K.rope(want[None, :, :H + Hk].cpu(), cos.cpu().double(), sin.cpu().double(), neox, pos0)[0].cuda()
+    got = x.clone()
+    N.check(N.lib().ptb_prompt_heads(got.data_ptr(), T, H, Hk, D, N.ptr(w[0]), N.ptr(w[1]), int(add_one), 1e-6, cos.data_ptr(), sin.data_ptr(), int(neox), pos0,
+                                     kc.data_ptr(), vc.data_ptr(), S, torch.cuda.current_stream().cuda_stream), "prompt_heads")
+    # one rounding: half a step of bf16 (eight significant bits: 2^-8 of a value at most) or fp16 (eleven: 2^-11), and fp32 arithmetic on values
+    # of the size of the head's largest
+    slack = 2 ** -20 * float(qk.abs().max())
+    assert bool(((got[:, :H + Hk].double() - qk).abs() <= 2 ** -8 * qk.abs() + slack).all())
+    assert torch.equal(got[:, H + Hk:], x[:, H + Hk:])
+    assert bool(((kc[:, pos0:pos0 + T].permute(1, 0, 2).double() - qk[:, H:]).abs() <= 2 ** -11 * qk[:, H:].abs() + 2 ** -24 + slack).all())
+    assert torch.equal(vc[:, pos0:pos0 + T].permute(1, 0, 2).float(), x[:, H + Hk:].half().float())
+    assert not bool(kc[:, :pos0].any()) and not bool(kc[:, pos0 + T:].any())
