@@ -2,6 +2,7 @@
 // resolved at run time, so the library loads on machines without a driver) and
 // the launcher that picks the tile width and operand majors.
 #include "gemm_sm100.cuh"
+#include "gemm_pair_sm100.cuh"
 #include <cudaTypedefs.h>
 #include <string.h>
 #include <algorithm>
@@ -157,10 +158,73 @@ static void fill_staging(Staging& S, const PtbStaging* h) {
 // `c_shards` fp32 buffers [out_shard_rows, ldc], one per rank.
 struct SplitK { int splits; long long stride; int bn; int pdl; };      // splits > 1: fp32 partials at C + s*stride; bn: 0 or a forced tile width
 
+// Whether a product runs on pairs of SMs, and how.  Times are in units of the pair kernel's k-block (256 x 256 x 64 on two SMs, about 0.33 us);
+// a 128 x 256 tile's k-block takes its one SM 1.3 of them and a 128 x 128 tile's 0.85 (measured over the products of the 2048- and
+// 4096-wide models, forward, both gradients: the ordinary kernels reach 500 to 1290 TFLOP/s, pairs 1070 to 1540), an epilogue about six, and
+// cut tiles a launch and their partials' bytes.  So the ordinary kernels keep what fills no more than one wave of their smaller tiles
+// (1024^3: 19.4 us against 21.5; 512 x 3072 x 2048: 27.7 against 29.7), and the last wave is cut where K is long: a weight gradient of
+// 2560 x 2048 over 8192 tokens 154 -> 66 us (uncut 92), of 1152 x 384 over 16384 132 -> 42 us (uncut 114).
+struct PairPlan { bool use; int whole, splits, kb_per_split; long long work_floats; };
+constexpr double T256 = 1.3, T128 = 0.85, EPI256 = 6.0, EPI128 = 4.0, PAIR_ITEM = 6.0, PAIR_LAUNCH = 2.0, PAIR_REDUCE = 8.0, PAIR_FLOAT = 5.6e-6;
+static PairPlan plan_pair(int M, int N, int K, int n_sm, bool may_cut) {
+    PairPlan best{false, 0, 1, 0, 0};
+    const int pairs = n_sm / 2;
+    if (M <= BM || pairs < 1) return best;
+    const int kb = (K + BK - 1) / BK;
+    const long long tm = (M + PAIR_M - 1) / PAIR_M, tn = (N + PAIR_N - 1) / PAIR_N, tiles = tm * tn;
+    auto waves = [](long long items, int per) { return (double)((items + per - 1) / per); };
+    const long long m128 = (M + 127) / 128;
+    const double t128 = waves(m128 * ((N + 127) / 128), n_sm) * (kb * T128 + EPI128), t256 = waves(m128 * ((N + 255) / 256), n_sm) * (kb * T256 + EPI256);
+    double cost = N > 128 ? std::min(t128, t256) : t128;
+    const long long rest = tiles % pairs;
+    for (int s = 1; s <= 32 && s <= kb; ++s) {
+        if (s > 1 && (!may_cut || rest == 0)) break;
+        const int kbps = (kb + s - 1) / s, real = (kb + kbps - 1) / kbps;
+        const long long whole = s == 1 ? tiles : tiles - rest, floats = s == 1 ? 0 : rest * real * PAIR_M * PAIR_N;
+        const double c = waves(whole, pairs) * (kb + PAIR_ITEM) + PAIR_LAUNCH +
+                         (s > 1 ? waves(rest * real, pairs) * (kbps + PAIR_ITEM) + PAIR_REDUCE + (double)floats * PAIR_FLOAT : 0.0);
+        if (c < cost) { cost = c; best = PairPlan{true, (int)whole, real, kbps, floats}; }
+    }
+    return best;
+}
+
+static int launch_pair(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C, long long ldc, int M, int N, int K, const float* bias,
+                       int flags, const PairPlan& plan, float* work, int* status, int n_sm, cudaStream_t st) {
+    CUtensorMap ma, mb;
+    if (ptb_make_tmap_bf16(&ma, A, a_mn ? M : K, a_mn ? K : M, lda, 64, a_mn ? 64 : 128)) return -1;
+    if (ptb_make_tmap_bf16(&mb, B, b_mn ? N : K, b_mn ? K : N, ldb, 64, b_mn ? 64 : 128)) return -1;
+    PairParams p;
+    memset(&p, 0, sizeof(p));
+    p.M = M; p.N = N; p.K = K; p.C = C; p.ldc = ldc; p.bias = bias; p.flags = flags; p.status = status;
+    p.tiles_m = (M + PAIR_M - 1) / PAIR_M;
+    p.tiles_n = (N + PAIR_N - 1) / PAIR_N;
+    p.whole = plan.whole; p.splits = plan.splits; p.kb_per_split = plan.kb_per_split; p.work = work;
+    p.pdl = !(flags & EPI_ACCUM) && ptb_pdl_enabled();
+    const int cut = p.tiles_m * p.tiles_n - p.whole;
+    const int pairs = std::max(1, std::min(n_sm / 2, p.whole + cut * p.splits));
+    static bool attr[4];
+    auto go = [&](auto kern) -> int {
+        bool& done = attr[(a_mn ? 2 : 0) + (b_mn ? 1 : 0)];
+        if (!done) {
+            PTB_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM));
+            done = true;
+        }
+        PTB_CUDA_OK(ptb_launch(kern, dim3(2 * pairs), dim3(THREADS), (size_t)PAIR_SMEM, st, p.pdl != 0, ma, mb, p));
+        if (cut > 0) PTB_CUDA_OK(ptb_launch(pair_reduce_kernel, dim3(cut * 8), dim3(256), 0, st, p.pdl != 0, p));
+        PTB_CUDA_OK(cudaGetLastError());
+        return 0;
+    };
+    if (!a_mn && !b_mn) return go(gemm_pair_kernel<false, false>);
+    if (!a_mn) return go(gemm_pair_kernel<false, true>);
+    if (!b_mn) return go(gemm_pair_kernel<true, false>);
+    return go(gemm_pair_kernel<true, true>);
+}
+
 static int gemm_core(void* const* a_ptrs, int a_shards, int a_shard_rows, long long lda, int a_mn, void* const* b_ptrs,
                      int b_shards, int b_shard_rows, long long ldb, int b_mn, void* C, long long ldc, void* const* c_peers,
                      int c_shards, int out_shard_rows, int M, int N, int K, const float* bias, int flags, int* status,
-                     int n_sm, cudaStream_t st, const PtbStaging* stage_a, const PtbStaging* stage_b, SplitK sk) {
+                     int n_sm, cudaStream_t st, const PtbStaging* stage_a, const PtbStaging* stage_b, SplitK sk, float* work = nullptr,
+                     long long work_floats = 0) {
     if (M <= 0 || N <= 0 || K <= 0) return 0;
     {
         int dev = 0;
@@ -187,6 +251,13 @@ static int gemm_core(void* const* a_ptrs, int a_shards, int a_shard_rows, long l
     } else {
         const int out_elem = (flags & EPI_OUT_F32) ? 4 : 2;
         if (((uintptr_t)C & 15) || ((ldc * out_elem) & 15)) { ptb_set_error("gemm: C needs a 16-byte aligned base and row pitch"); return -1; }
+    }
+    // a plain product of local operands
+    if (!(flags & (EPI_SCATTER_ADD | EPI_SCATTER_STORE | EPI_TRANS)) && a_shards == 1 && b_shards == 1 && !sk.bn && sk.splits <= 1 &&
+        !(stage_a && stage_a->seq) && !(stage_b && stage_b->seq)) {
+        PairPlan plan = plan_pair(M, N, K, n_sm, work != nullptr);
+        if (plan.use && plan.work_floats > work_floats) plan = plan_pair(M, N, K, n_sm, false);
+        if (plan.use) return launch_pair(a_ptrs[0], lda, a_mn, b_ptrs[0], ldb, b_mn, C, ldc, M, N, K, bias, flags, plan, work, status, n_sm, st);
     }
     int BN = N > 128 ? 256 : 128;
     if (BN == 256) {
@@ -555,3 +626,16 @@ PTB_API int ptb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B,
     void* bp[1] = {const_cast<void*>(B)};
     return ptb_gemm_bf16_ex(ap, 1, 0, lda, a_mn, bp, 1, 0, ldb, b_mn, C, ldc, nullptr, 0, 0, M, N, K, bias, flags, status, n_sm, st, nullptr, nullptr);
 }
+
+// Floats of workspace with which ptb_gemm_bf16_ws cuts the tiles of the last wave along K (0: it would not).
+PTB_API long long ptb_gemm_work_floats(int M, int N, int K, int n_sm) { return plan_pair(M, N, K, n_sm, true).work_floats; }
+
+// The same with a workspace of `work_floats` floats (16-byte aligned) for partial sums.
+PTB_API int ptb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C, long long ldc, int M, int N, int K,
+                             const float* bias, int flags, float* work, long long work_floats, int* status, int n_sm, cudaStream_t st) {
+    void* ap[1] = {const_cast<void*>(A)};
+    void* bp[1] = {const_cast<void*>(B)};
+    return gemm_core(ap, 1, 0, lda, a_mn, bp, 1, 0, ldb, b_mn, C, ldc, nullptr, 0, 0, M, N, K, bias, flags, status, n_sm, st, nullptr, nullptr, SplitK{1, 0, 0, 0},
+                     ((uintptr_t)work & 15) ? nullptr : work, work_floats);
+}
+

@@ -23,6 +23,10 @@ def _decls(L):
     vp, ci, ll = C.c_void_p, C.c_int, C.c_longlong
     L.ptb_gemm_bf16.argtypes = [vp, ll, ci, vp, ll, ci, vp, ll, ci, ci, ci, vp, ci, vp, ci, vp]
     L.ptb_gemm_bf16.restype = ci
+    L.ptb_gemm_work_floats.argtypes = [ci, ci, ci, ci]
+    L.ptb_gemm_work_floats.restype = ll
+    L.ptb_gemm_bf16_ws.argtypes = [vp, ll, ci, vp, ll, ci, vp, ll, ci, ci, ci, vp, ci, vp, ll, vp, ci, vp]
+    L.ptb_gemm_bf16_ws.restype = ci
     if hasattr(L, "ptb_gemm_bf16_splitk"):
         L.ptb_gemm_pick_splits.argtypes = [ci, ci, ci, ci]
         L.ptb_gemm_pick_splits.restype = ci
@@ -101,8 +105,10 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
     if bias is not None:
         bias = bias.float().contiguous()
     st = torch.cuda.current_stream(a.device).cuda_stream
-    N.check(N.lib().ptb_gemm_bf16(a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn), out.data_ptr(),
-                                  out.stride(0), M, Nn, K, N.ptr(bias), flags, _status(a.device).data_ptr(), 0, st), "gemm_bf16")
+    floats = int(N.lib().ptb_gemm_work_floats(M, Nn, K, _sms(a.device)))        # partials of the last wave's tiles, where cutting them pays
+    work = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
+    N.check(N.lib().ptb_gemm_bf16_ws(a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn), out.data_ptr(), out.stride(0), M, Nn, K,
+                                     N.ptr(bias), flags, N.ptr(work), floats, _status(a.device).data_ptr(), 0, st), "gemm_bf16")
     return out
 
 
