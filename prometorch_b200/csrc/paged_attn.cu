@@ -5,9 +5,9 @@
 // tensor per layer, [page][kv_head][64][D]; a step of the engine serves every active request in one batch:
 //   paged_rope_write_kernel  rotates q (in place) and k of the new tokens and stores k, v in the slot the page
 //                            table gives for (request, position);
-//   paged_attn_decode_kernel one CTA per (kv head, request, split): its warps walk the request's pages with an
-//                            online softmax for the whole GQA group, merge through shared memory, and either
-//                            finish or leave a partial (max, sum, acc) for paged_attn_merge_kernel.
+//   paged_attn_decode_kernel one CTA per (kv head, request, split): its warps walk the split's tokens with an
+//                            online softmax for the whole GQA group, merge through shared memory and across the cluster of
+//                            the splits, or leave a partial (max, sum, acc) for paged_attn_merge_kernel.
 // A page id outside the pool is never dereferenced: the kernel records PTB_ERR_BOUNDS and skips the page.
 #include "common.cuh"
 #include <algorithm>
@@ -15,7 +15,8 @@
 namespace ptb {
 
 constexpr int PAGE = 64;
-constexpr int PA_WARPS = 4;
+constexpr int PA_WARPS = 8;
+constexpr int PA_CLUSTER = 16;           // splits that merge within a cluster (more than eight need the attribute below)
 constexpr int PA_THREADS = PA_WARPS * 32;
 
 struct PagedWriteParams {
@@ -93,16 +94,38 @@ __global__ void __launch_bounds__(256) paged_rope_write_kernel(const __grid_cons
     }
 }
 
-// The same for projections in bf16 with 16-byte rows: a thread rotates eight pairs (two 16-byte loads, D/16 threads a head) or moves eight
+// The same in 16-byte pieces, for bf16 rows or (PARTS) split-K partials: a thread rotates eight pairs (two 16-byte loads, D/16 threads a head) or moves eight
 // values.  What bounds it is bytes: each value is read once and written once or twice.  One CTA per token either way; two bytes
 // an access it cost the 8-request, 14192-token prompt pass of a 4096-wide model (8 layers, then 16 tokens each) 88.4 ms in place of 84.2.
+template <bool PARTS>
 __global__ void __launch_bounds__(256) paged_rope_write_vec_kernel(const __grid_constant__ PagedWriteParams P) {
     pdl_wait();
     pdl_launch_dependents();
     const int i = blockIdx.x;
     const int half = P.D / 2, per_half = half / 8, per_head = P.D / 8;
     const int pos = P.pos[i];
-    uint4* row = reinterpret_cast<uint4*>(P.qkv + (size_t)i * (P.H + 2 * P.Hk) * P.D);
+    const size_t width = (size_t)(P.H + 2 * P.Hk) * P.D;
+    uint4* row = PARTS ? nullptr : reinterpret_cast<uint4*>(P.qkv + i * width);
+    // eight neighbouring values of the projection, from 16-byte piece `at` on
+    auto load8 = [&](int at, float* f) {
+        if constexpr (PARTS) {
+            const float4* w = reinterpret_cast<const float4*>(P.work + i * width) + 2 * at;
+            float4 a = w[0], b = w[1];
+#pragma unroll 4
+            for (int s = 1; s < P.splits; ++s) {
+                const float4* ws = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(w) + (size_t)s * P.split_stride);
+                const float4 c = ws[0], d = ws[1];
+                a.x += c.x; a.y += c.y; a.z += c.z; a.w += c.w;
+                b.x += d.x; b.y += d.y; b.z += d.z; b.w += d.w;
+            }
+            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        } else {
+            const uint4 raw = row[at];
+            const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+            for (int x = 0; x < 4; ++x) { const float2 v = __bfloat1622float2(h2[x]); f[2 * x] = v.x; f[2 * x + 1] = v.y; }
+        }
+    };
     const int page_slot = pos / PAGE, in_page = pos % PAGE;
     const int page = P.page_table[(size_t)P.req[i] * P.pt_stride + max(0, min(page_slot, P.pt_stride - 1))];
     const bool ok = pos >= 0 && pos < P.max_pos && page_slot < P.pt_stride && page >= 0 && page < P.n_pages;
@@ -118,19 +141,21 @@ __global__ void __launch_bounds__(256) paged_rope_write_vec_kernel(const __grid_
     for (int e = threadIdx.x; e < n_all; e += 256) {
         if (e < n_rot) {
             const int h = e / per_half, j = e - h * per_half;
-            const uint4 lo = row[h * per_head + j], hi = row[h * per_head + per_half + j];
+            float lo[8], hi[8];
+            load8(h * per_head + j, lo);
+            load8(h * per_head + per_half + j, hi);
             const float4 c0 = cs[2 * j], c1 = cs[2 * j + 1], s0 = sn[2 * j], s1 = sn[2 * j + 1];
             const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, s[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-            const __nv_bfloat162 *a2 = reinterpret_cast<const __nv_bfloat162*>(&lo), *b2 = reinterpret_cast<const __nv_bfloat162*>(&hi);
             uint4 ra, rb;
             __nv_bfloat162 *oa = reinterpret_cast<__nv_bfloat162*>(&ra), *ob = reinterpret_cast<__nv_bfloat162*>(&rb);
 #pragma unroll
             for (int x = 0; x < 4; ++x) {
-                const float2 a = __bfloat1622float2(a2[x]), b = __bfloat1622float2(b2[x]);
+                const float2 a = make_float2(lo[2 * x], lo[2 * x + 1]), b = make_float2(hi[2 * x], hi[2 * x + 1]);
                 oa[x] = __floats2bfloat162_rn(a.x * c[2 * x] - b.x * s[2 * x], a.y * c[2 * x + 1] - b.y * s[2 * x + 1]);
                 ob[x] = __floats2bfloat162_rn(b.x * c[2 * x] + a.x * s[2 * x], b.y * c[2 * x + 1] + a.y * s[2 * x + 1]);
             }
-            uint4* dst = h < P.H ? row + h * per_head : slot(P.k_pages, h - P.H);
+            uint4* q_row = PARTS ? reinterpret_cast<uint4*>(P.q_out + (size_t)i * P.H * P.D) : row;
+            uint4* dst = h < P.H ? q_row + h * per_head : slot(P.k_pages, h - P.H);
             dst[j] = ra; dst[per_half + j] = rb;
             if (h >= P.H && P.k_out) {
                 uint4* ko = reinterpret_cast<uint4*>(P.k_out + ((size_t)i * P.Hk + h - P.H) * P.D);
@@ -138,7 +163,17 @@ __global__ void __launch_bounds__(256) paged_rope_write_vec_kernel(const __grid_
             }
         } else {
             const int c = e - n_rot, kh = c / per_head, d = c - kh * per_head;
-            slot(P.v_pages, kh)[d] = row[(P.H + P.Hk) * per_head + c];
+            if constexpr (PARTS) {
+                float f[8];
+                load8((P.H + P.Hk) * per_head + c, f);
+                uint4 o;
+                __nv_bfloat162* oh = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+                for (int x = 0; x < 4; ++x) oh[x] = __floats2bfloat162_rn(f[2 * x], f[2 * x + 1]);
+                slot(P.v_pages, kh)[d] = o;
+            } else {
+                slot(P.v_pages, kh)[d] = row[(P.H + P.Hk) * per_head + c];
+            }
         }
     }
 }
@@ -155,130 +190,150 @@ struct PagedAttnParams {
     float* work;                   // [B, H, nsplit, D + 2] partial (acc, max, sum) when nsplit > 1
     int B, H, Hk, nsplit;
     float scale_log2;              // softmax scale times log2(e)
+    int q_wide;                    // rows of q start on 16 bytes
+    int cluster;                   // the splits of a (kv head, request) are a cluster
     int* status;
 };
 
+__device__ __forceinline__ void unpack8(const uint4& raw, float* f) {
+    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 v = __bfloat1622float2(h2[i]); f[2 * i] = v.x; f[2 * i + 1] = v.y; }
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
+    float v;
+    asm volatile("{\n .reg .b32 a;\n mapa.shared::cluster.u32 a, %1, %2;\n ld.shared::cluster.f32 %0, [a];\n}" : "=f"(v) : "r"(addr), "r"(rank) : "memory");
+    return v;
+}
+__device__ __forceinline__ void pa_cluster_sync() { asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// D / 8 lanes a token, eight values a lane: a warp's load covers whole rows, K and V of its group of TG tokens are requested together, and its
+// online softmax needs no other warp until the end.  Bound by the cache's bytes at long contexts and by latency at short ones, so
+// tokens, not pages, are dealt to warps: one lane per token and one warp per page had nine warps work on a request of 540 tokens
+// (per kv head of 128, groups of 4: 27 us, and 3 for the merge).  Up to sixteen splits are the CTAs of a cluster, which merge through
+// distributed shared memory; more leave partials for paged_attn_merge_kernel.
 template <int D, int G>
-__global__ void __launch_bounds__(PA_THREADS, (G <= 4 ? 8 : 6)) paged_attn_decode_kernel(const __grid_constant__ PagedAttnParams P) {
-    constexpr int DV = D / 32;                        // output dims per lane (4 or 2)
-    static_assert(DV == 4 || DV == 2, "head size 128 or 64");
-    __shared__ float q_s[G][D];
-    __shared__ float p_s[PA_WARPS][G][PAGE];
-    __shared__ float acc_s[PA_WARPS][G][D];
+__global__ void __launch_bounds__(PA_THREADS, G == 8 ? 1 : 2) paged_attn_decode_kernel(const __grid_constant__ PagedAttnParams P) {
+    constexpr int LPT = D / 8, TPI = 32 / LPT, U = G == 8 ? 2 : 4, TG = TPI * U;
+    static_assert(D == 128 || D == 64, "head size 128 or 64");
+    static_assert(PAGE % TG == 0, "a group lies in one page");
+    __shared__ __align__(16) float acc_s[PA_WARPS][G][D];
     __shared__ float ml_s[PA_WARPS][G][2];
+    __shared__ float part[G * D], part_ml[2 * G];
     const int kvh = blockIdx.x, b = blockIdx.y, split = blockIdx.z;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPT, l = lane % LPT;
     pdl_wait();
     pdl_launch_dependents();
-    for (int e = threadIdx.x; e < G * D; e += PA_THREADS) {
-        const int g = e / D, d = e % D;
-        q_s[g][d] = __bfloat162float(P.q[(size_t)b * P.q_stride + (size_t)(kvh * G + g) * D + d]) * P.scale_log2;
+    uint4 qr[G];
+    {
+        const __nv_bfloat16* qp = P.q + (size_t)b * P.q_stride + (size_t)kvh * G * D + l * 8;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (P.q_wide) {
+                qr[g] = *reinterpret_cast<const uint4*>(qp + g * D);
+            } else {
+                __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&qr[g]);
+#pragma unroll
+                for (int i = 0; i < 8; ++i) e[i] = qp[g * D + i];
+            }
+        }
     }
-    __syncthreads();
-    const int len = P.lens[b];
-    const int npages = min((len + PAGE - 1) / PAGE, P.pt_stride);
-    // pages of this split, dealt to the warps round-robin
-    const int per = (npages + P.nsplit - 1) / P.nsplit;
-    const int p_lo = split * per, p_hi = min(p_lo + per, npages);
-    float m[G], l[G], acc[G][DV];
+    const int len = min(P.lens[b], P.pt_stride * PAGE);
+    // tokens of this split, in groups dealt to the warps round-robin
+    const int per = ((len + P.nsplit - 1) / P.nsplit + TG - 1) / TG * TG;
+    const int lo = split * per, hi = min(lo + per, len);
+    float m[G], sum[G], acc[G][8];
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        m[g] = -INFINITY; l[g] = 0.f;
+        m[g] = -INFINITY; sum[g] = 0.f;
 #pragma unroll
-        for (int i = 0; i < DV; ++i) acc[g][i] = 0.f;
+        for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
     }
-    for (int pg = p_lo + warp; pg < p_hi; pg += PA_WARPS) {
-        const int page = P.page_table[(size_t)b * P.pt_stride + pg];
+    for (int t0 = lo + warp * TG; t0 < hi; t0 += PA_WARPS * TG) {
+        const int page = P.page_table[(size_t)b * P.pt_stride + t0 / PAGE];
         if (page < 0 || page >= P.n_pages) {
             if (lane == 0 && P.status) atomicExch(P.status, PTB_ERR_BOUNDS);
             continue;
         }
-        const int valid = min(PAGE, len - pg * PAGE);
-        const __nv_bfloat16* kb = P.k_pages + ((size_t)page * P.Hk + kvh) * PAGE * D;
-        const __nv_bfloat16* vb = P.v_pages + ((size_t)page * P.Hk + kvh) * PAGE * D;
-        // scores: each lane owns tokens lane and lane + 32 and walks their rows in 16-byte pieces
-        float s[2][G];
+        const size_t at = (((size_t)page * P.Hk + kvh) * PAGE + t0 % PAGE + sub) * D + l * 8;
+        uint4 kr[U], vr[U];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            const int t = lane + r * 32;
+        for (int u = 0; u < U; ++u) kr[u] = *reinterpret_cast<const uint4*>(P.k_pages + at + (size_t)u * TPI * D);
 #pragma unroll
-            for (int g = 0; g < G; ++g) s[r][g] = 0.f;
-            if (t < valid) {
-                const uint4* kr = reinterpret_cast<const uint4*>(kb + (size_t)t * D);
-#pragma unroll 8
-                for (int c = 0; c < D / 8; ++c) {
-                    const uint4 raw = kr[c];
-                    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
-                    float kf[8];
+        for (int u = 0; u < U; ++u) vr[u] = *reinterpret_cast<const uint4*>(P.v_pages + at + (size_t)u * TPI * D);
+        float s[U][G];
+        {
+            float kf[U][8];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h2[i]); kf[2 * i] = f.x; kf[2 * i + 1] = f.y; }
+            for (int u = 0; u < U; ++u) unpack8(kr[u], kf[u]);
 #pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const float4 qa = *reinterpret_cast<const float4*>(&q_s[g][c * 8]);
-                        const float4 qb = *reinterpret_cast<const float4*>(&q_s[g][c * 8 + 4]);
-                        s[r][g] += qa.x * kf[0] + qa.y * kf[1] + qa.z * kf[2] + qa.w * kf[3] + qb.x * kf[4] + qb.y * kf[5] + qb.z * kf[6] + qb.w * kf[7];
-                    }
+            for (int g = 0; g < G; ++g) {
+                float qf[8];
+                unpack8(qr[g], qf);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    float d0 = qf[0] * kf[u][0], d1 = qf[1] * kf[u][1];
+#pragma unroll
+                    for (int i = 2; i < 8; i += 2) { d0 += qf[i] * kf[u][i]; d1 += qf[i + 1] * kf[u][i + 1]; }
+                    s[u][g] = d0 + d1;
                 }
-            } else {
-#pragma unroll
-                for (int g = 0; g < G; ++g) s[r][g] = -INFINITY;
             }
+        }
+#pragma unroll
+        for (int o = LPT / 2; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int g = 0; g < G; ++g) s[u][g] += __shfl_xor_sync(0xffffffffu, s[u][g], o);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = t0 + u * TPI + sub < len;
+#pragma unroll
+            for (int g = 0; g < G; ++g) s[u][g] = in ? s[u][g] * P.scale_log2 : -INFINITY;
+            if (!in) vr[u] = make_uint4(0, 0, 0, 0);
         }
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            const float mx = warp_max(fmaxf(s[0][g], s[1][g]));
-            const float m_new = fmaxf(m[g], mx);                       // finite: a page always has a valid token
-            const float corr = exp2f(m[g] - m_new);
-            const float p0 = exp2f(s[0][g] - m_new), p1 = exp2f(s[1][g] - m_new);
-            p_s[warp][g][lane] = p0;
-            p_s[warp][g][lane + 32] = p1;
-            l[g] = l[g] * corr + warp_sum(p0 + p1);
+            float mx = s[0][g];
+#pragma unroll
+            for (int u = 1; u < U; ++u) mx = fmaxf(mx, s[u][g]);
+#pragma unroll
+            for (int o = LPT; o < 32; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+            const float m_new = fmaxf(m[g], mx), m_use = m_new == -INFINITY ? 0.f : m_new;
+            const float corr = exp2f(m[g] - m_use);
+            float add = 0.f;
+#pragma unroll
+            for (int u = 0; u < U; ++u) { s[u][g] = exp2f(s[u][g] - m_use); add += s[u][g]; }
+            sum[g] = sum[g] * corr + add;                       // of this lane's tokens
             m[g] = m_new;
 #pragma unroll
-            for (int i = 0; i < DV; ++i) acc[g][i] *= corr;
+            for (int i = 0; i < 8; ++i) acc[g][i] *= corr;
         }
-        __syncwarp();
-        // P V: each lane owns DV consecutive output dims.  Sixteen rows are fetched (kept packed) before they are used so
-        // that sixteen loads are in flight per lane; rows past `valid` belong to the page (readable) and carry p = 0.
-        constexpr int PF = 16;
-        for (int t0 = 0; t0 < valid; t0 += PF) {
-            if constexpr (DV == 4) {
-                uint2 raw[PF];
 #pragma unroll
-                for (int u = 0; u < PF; ++u) raw[u] = *reinterpret_cast<const uint2*>(vb + (size_t)(t0 + u) * D + lane * 4);
+        for (int u = 0; u < U; ++u) {
+            float vf[8];
+            unpack8(vr[u], vf);
 #pragma unroll
-                for (int u = 0; u < PF; ++u) {
-                    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw[u]);
-                    const float2 a = __bfloat1622float2(h2[0]), c = __bfloat1622float2(h2[1]);
+            for (int g = 0; g < G; ++g)
 #pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const float p = p_s[warp][g][t0 + u];
-                        acc[g][0] += p * a.x; acc[g][1] += p * a.y; acc[g][2] += p * c.x; acc[g][3] += p * c.y;
-                    }
-                }
-            } else {
-                uint32_t raw[PF];
-#pragma unroll
-                for (int u = 0; u < PF; ++u) raw[u] = *reinterpret_cast<const uint32_t*>(vb + (size_t)(t0 + u) * D + lane * 2);
-#pragma unroll
-                for (int u = 0; u < PF; ++u) {
-                    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw[u]));
-#pragma unroll
-                    for (int g = 0; g < G; ++g) {
-                        const float p = p_s[warp][g][t0 + u];
-                        acc[g][0] += p * a.x; acc[g][1] += p * a.y;
-                    }
-                }
-            }
+                for (int i = 0; i < 8; ++i) acc[g][i] += s[u][g] * vf[i];
         }
-        __syncwarp();
     }
-    // merge the warps
+    // the lanes that hold the same values of different tokens, then the warps
 #pragma unroll
     for (int g = 0; g < G; ++g) {
 #pragma unroll
-        for (int i = 0; i < DV; ++i) acc_s[warp][g][lane * DV + i] = acc[g][i];
-        if (lane == 0) { ml_s[warp][g][0] = m[g]; ml_s[warp][g][1] = l[g]; }
+        for (int o = LPT; o < 32; o <<= 1) {
+            sum[g] += __shfl_xor_sync(0xffffffffu, sum[g], o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) acc[g][i] += __shfl_xor_sync(0xffffffffu, acc[g][i], o);
+        }
+        if (sub == 0) {
+            float4* dst = reinterpret_cast<float4*>(&acc_s[warp][g][l * 8]);
+            dst[0] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+            dst[1] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
+        }
+        if (lane == 0) { ml_s[warp][g][0] = m[g]; ml_s[warp][g][1] = sum[g]; }
     }
     __syncthreads();
     for (int e = threadIdx.x; e < G * D; e += PA_THREADS) {
@@ -293,15 +348,34 @@ __global__ void __launch_bounds__(PA_THREADS, (G <= 4 ? 8 : 6)) paged_attn_decod
             L += ml_s[w][g][1] * f;
             o += acc_s[w][g][d] * f;
         }
-        const int h = kvh * G + g;
         if (P.nsplit == 1) {
-            P.out[((size_t)b * P.H + h) * D + d] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+            P.out[((size_t)b * P.H + kvh * G + g) * D + d] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+        } else if (P.cluster) {
+            part[e] = o;
+            if (d == 0) { part_ml[g] = M; part_ml[G + g] = L; }
         } else {
-            float* wk = P.work + (((size_t)b * P.H + h) * P.nsplit + split) * (D + 2);
+            float* wk = P.work + (((size_t)b * P.H + kvh * G + g) * P.nsplit + split) * (D + 2);
             wk[d] = o;
             if (d == 0) { wk[D] = M; wk[D + 1] = L; }
         }
     }
+    if (!P.cluster) return;
+    // split r of the cluster finishes every nsplit-th output
+    pa_cluster_sync();
+    const uint32_t a_part = smem_u32(part), a_ml = smem_u32(part_ml);
+    for (int e = threadIdx.x * P.nsplit + split; e < G * D; e += PA_THREADS * P.nsplit) {
+        const int g = e / D;
+        float M = -INFINITY, L = 0.f, o = 0.f;
+        for (int r = 0; r < P.nsplit; ++r) M = fmaxf(M, ld_cluster_f32(a_ml + g * 4, r));
+        for (int r = 0; r < P.nsplit; ++r) {
+            const float mr = ld_cluster_f32(a_ml + g * 4, r);
+            const float f = mr == -INFINITY ? 0.f : exp2f(mr - M);
+            L += ld_cluster_f32(a_ml + (G + g) * 4, r) * f;
+            o += ld_cluster_f32(a_part + e * 4, r) * f;
+        }
+        P.out[((size_t)b * P.H + kvh * G + g) * D + e % D] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
+    }
+    pa_cluster_sync();                             // the others may still read this CTA's part
 }
 
 // Combine the splits of one (request, head): grid (H, B), D threads.
@@ -322,16 +396,42 @@ __global__ void paged_attn_merge_kernel(const float* __restrict__ work, __nv_bfl
     out[((size_t)b * H + h) * D + d] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
 }
 
+template <int D, int G>
+static cudaError_t launch_decode_g(const PagedAttnParams& p, cudaStream_t st) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(p.Hk, p.B, p.nsplit);
+    cfg.blockDim = dim3(PA_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (ptb_pdl_enabled()) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (p.cluster) {
+        static bool wide = false;
+        if (p.nsplit > 8 && !wide) {
+            const cudaError_t e = cudaFuncSetAttribute(paged_attn_decode_kernel<D, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            if (e != cudaSuccess) return e;
+            wide = true;
+        }
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = 1; attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = (unsigned)p.nsplit;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    return cudaLaunchKernelEx(&cfg, paged_attn_decode_kernel<D, G>, p);
+}
+
 template <int D>
 static int launch_decode(const PagedAttnParams& p, int G, cudaStream_t st) {
-    dim3 grid(p.Hk, p.B, p.nsplit);
-    const bool pdl = ptb_pdl_enabled();
     cudaError_t e;
     switch (G) {
-        case 1: e = ptb_launch(paged_attn_decode_kernel<D, 1>, grid, dim3(PA_THREADS), 0, st, pdl, p); break;
-        case 2: e = ptb_launch(paged_attn_decode_kernel<D, 2>, grid, dim3(PA_THREADS), 0, st, pdl, p); break;
-        case 4: e = ptb_launch(paged_attn_decode_kernel<D, 4>, grid, dim3(PA_THREADS), 0, st, pdl, p); break;
-        case 8: e = ptb_launch(paged_attn_decode_kernel<D, 8>, grid, dim3(PA_THREADS), 0, st, pdl, p); break;
+        case 1: e = launch_decode_g<D, 1>(p, st); break;
+        case 2: e = launch_decode_g<D, 2>(p, st); break;
+        case 4: e = launch_decode_g<D, 4>(p, st); break;
+        case 8: e = launch_decode_g<D, 8>(p, st); break;
         default: ptb_set_error("paged attention: group size %d not in {1, 2, 4, 8}", G); return -1;
     }
     PTB_CUDA_OK(e);
@@ -354,10 +454,11 @@ static int rope_write(void* qkv, const float* work, int splits, void* q_out, int
     p.qkv = (__nv_bfloat16*)qkv; p.pos = pos; p.req = req; p.page_table = page_table; p.pt_stride = pt_stride; p.n_pages = n_pages;
     p.cos = cos; p.sin = sin; p.k_pages = (__nv_bfloat16*)k_pages; p.v_pages = (__nv_bfloat16*)v_pages; p.k_out = (__nv_bfloat16*)k_out;
     p.n = n; p.H = H; p.Hk = Hk; p.D = D; p.max_pos = max_pos; p.status = status;
-    // rows of a bf16 projection in 16-byte pieces: half a head is a multiple of eight values and every base is aligned (a head then is too)
-    const bool vec = !work && D % 16 == 0 &&
-                     !(((uintptr_t)qkv | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)k_out | (uintptr_t)cos | (uintptr_t)sin) & 15);
-    PTB_CUDA_OK(ptb_launch(vec ? paged_rope_write_vec_kernel : paged_rope_write_kernel, dim3(n), dim3(256), 0, st, ptb_pdl_enabled(), p));
+    // 16-byte pieces: half a head is a multiple of eight values and every base is aligned (a head then is too)
+    const bool vec = D % 16 == 0 && !(((uintptr_t)qkv | (uintptr_t)work | (uintptr_t)q_out | (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)k_out | (uintptr_t)cos |
+                                       (uintptr_t)sin) & 15);
+    PTB_CUDA_OK(ptb_launch(!vec ? paged_rope_write_kernel : work ? paged_rope_write_vec_kernel<true> : paged_rope_write_vec_kernel<false>, dim3(n), dim3(256), 0, st,
+                           ptb_pdl_enabled(), p));
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }
@@ -379,8 +480,8 @@ PTB_API int ptb_paged_rope_write_partials(const float* work, int splits, void* q
                       nullptr, status, st);
 }
 
-// Floats of workspace ptb_paged_attn_decode needs for `nsplit` > 1.
-PTB_API long long ptb_paged_attn_work_floats(int B, int H, int D, int nsplit) { return nsplit > 1 ? (long long)B * H * nsplit * (D + 2) : 0; }
+// Floats of workspace ptb_paged_attn_decode needs (up to sixteen splits merge on the chip).
+PTB_API long long ptb_paged_attn_work_floats(int B, int H, int D, int nsplit) { return nsplit > PA_CLUSTER ? (long long)B * H * nsplit * (D + 2) : 0; }
 
 // One new token per request attends to its pages.  q: [B, q_stride] bf16; out: [B, H D] bf16; lens: [B].
 PTB_API int ptb_paged_attn_decode(const void* q, long long q_stride, void* out, int B, int H, int Hk, int D, const int* lens,
@@ -388,17 +489,19 @@ PTB_API int ptb_paged_attn_decode(const void* q, long long q_stride, void* out, 
                                   float scale, float* work, int nsplit, int* status, cudaStream_t st) {
     if (B <= 0) return 0;
     if (Hk <= 0 || H % Hk) { ptb_set_error("paged attention: %d heads over %d kv heads", H, Hk); return -1; }
-    if (nsplit < 1 || (nsplit > 1 && !work)) { ptb_set_error("paged attention: nsplit %d needs a workspace", nsplit); return -1; }
+    if (nsplit < 1 || (nsplit > PA_CLUSTER && !work)) { ptb_set_error("paged attention: nsplit %d needs a workspace", nsplit); return -1; }
     PagedAttnParams p;
     p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride; p.out = (__nv_bfloat16*)out; p.lens = lens; p.page_table = page_table;
     p.pt_stride = pt_stride; p.n_pages = n_pages; p.k_pages = (const __nv_bfloat16*)k_pages; p.v_pages = (const __nv_bfloat16*)v_pages;
     p.work = work; p.B = B; p.H = H; p.Hk = Hk; p.nsplit = nsplit; p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
+    p.cluster = nsplit > 1 && nsplit <= PA_CLUSTER;
+    p.q_wide = !((uintptr_t)q & 15) && q_stride % 8 == 0;
     int rc;
     if (D == 128) rc = launch_decode<128>(p, H / Hk, st);
     else if (D == 64) rc = launch_decode<64>(p, H / Hk, st);
     else { ptb_set_error("paged attention: head size %d not in {64, 128}", D); return -1; }
     if (rc) return rc;
-    if (nsplit > 1)
+    if (nsplit > PA_CLUSTER)
         PTB_CUDA_OK(ptb_launch(paged_attn_merge_kernel, dim3(H, B), dim3(D), 0, st, ptb_pdl_enabled(), (const float*)work, (__nv_bfloat16*)out, H, D, nsplit));
     PTB_CUDA_OK(cudaGetLastError());
     return 0;

@@ -188,7 +188,8 @@ class PagedLlama(PagedModel):
         x = w.tok_emb[ids]
         h = self._norm(x, w.layers[0]["attn_norm"])
         for l, L in enumerate(w.layers):
-            q = P.qkv_rope_write(h, L["wqkv"], H, Hk, Dh, pos, req, table, self.cos, self.sin, kv.k[l], kv.v[l])
+            q = P.qkv_rope_write(h, L["wqkv"], H, Hk, Dh, pos, req, table, self.cos, self.sin, kv.k[l], kv.v[l],
+                                 fuse_sum=True)
             a = P.paged_attention_decode(q, H, Hk, Dh, lens, table, kv.k[l], kv.v[l], nsplit=nsplit)
             h, x = linear_add_rms_norm(a, L["wo"], x, L["ffn_norm"], c.rms_norm_eps)
             nxt = w.layers[l + 1]["attn_norm"] if l + 1 < len(w.layers) else w.final_norm

@@ -97,11 +97,9 @@ def paged_rope_write(qkv: torch.Tensor, H: int, Hk: int, D: int, pos: torch.Tens
 
 def qkv_rope_write(h: torch.Tensor, wqkv: torch.Tensor, H: int, Hk: int, D: int, pos, req, page_table, cos, sin, k_pages, v_pages,
                    fuse_sum: bool = False):
-    """``qkv = h Wqkv^T`` followed by :func:`paged_rope_write`; returns a tensor whose first ``H D`` columns are the rotated q.  For
-    decode-sized CUDA batches the projection stays as split-K partials and the rotary kernel sums them while it
-    reads (no reduce launch, no bf16 round trip of k and v) when ``fuse_sum`` is set.  That is off by default: the
-    rotary kernel is one CTA per token and sums the partials with scalar loads, and the decode pass of the 16-layer
-    2048-wide model measured 1.24 ms with it against 1.15 ms with the separate, vectorised reduce launch."""
+    """``qkv = h Wqkv^T`` followed by :func:`paged_rope_write`; returns a tensor whose first ``H D`` columns are the rotated q.  With ``fuse_sum``
+    the projection of a decode-sized CUDA batch stays as split-K partials and the rotary kernel sums them while it reads: no
+    reduce launch, no bf16 round trip of q, k and v."""
     from .gemm import _skinny_splits, _status as gemm_status, linear
     splits = _skinny_splits(h, wqkv) if h.is_cuda else 0
     if fuse_sum and splits and hasattr(N.lib(), "ptb_paged_rope_write_partials") and not torch.is_grad_enabled():
@@ -123,14 +121,18 @@ def qkv_rope_write(h: torch.Tensor, wqkv: torch.Tensor, H: int, Hk: int, D: int,
 
 
 def pick_splits(B: int, Hk: int, max_len: int, sms: int = 148) -> int:
-    """Splits of the page walk.  A CTA is four warps with a few KB of loads in flight each, so the kernel wants about
-    eight CTAs per SM to saturate HBM; a split should still own two pages or more.  The page count is rounded up to a
-    power of two so that the choice (a key of the engine's graph cache) changes rarely as a context grows."""
+    """Splits of the page walk, each a CTA of eight warps and of at least a page; a power of two (the choice is a key of the engine's graph
+    cache, so it should change rarely).  Splits pay until every SM has a CTA, and beyond that only where each keeps a long walk: launching
+    and merging clusters costs more than idle SMs.  Measured, us: 1 request, 4 kv heads, 540 tokens: 12.0 (1 split), 6.2 (16); 32 requests, 4 heads of a
+    group of 4, 300 tokens: 8.4 (1), 9.2 (2), 25.3 (8), 1500 tokens: 36.7 (1), 29.6 (2), 45.9 (8); 8 requests, 32 heads, 1800 tokens: 42.3 (1), 49.6 (2)."""
     pages = max(1, (max_len + PAGE - 1) // PAGE)
-    bucket = 1
-    while bucket < pages:
-        bucket *= 2
-    return int(max(1, min(16, bucket // 2, (8 * sms) // max(1, B * Hk))))
+    n = 1
+    while n < 16 and n < pages:
+        ctas, each = 2 * n * B * Hk, max_len // (2 * n)
+        if not (ctas <= sms or (ctas <= 2 * sms and each >= 512) or (ctas <= 8 * sms and each >= 4096)):
+            break
+        n *= 2
+    return n
 
 
 def paged_attention_decode(q: torch.Tensor, H: int, Hk: int, D: int, lens: torch.Tensor, page_table: torch.Tensor,
@@ -142,8 +144,8 @@ def paged_attention_decode(q: torch.Tensor, H: int, Hk: int, D: int, lens: torch
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     if _cuda_ok(q) and D in (64, 128) and H // Hk in (1, 2, 4, 8):
         out = torch.empty(B, H * D, dtype=q.dtype, device=q.device)
-        work = torch.empty(int(N.lib().ptb_paged_attn_work_floats(B, H, D, nsplit)), dtype=torch.float32, device=q.device) \
-            if nsplit > 1 else None
+        floats = int(N.lib().ptb_paged_attn_work_floats(B, H, D, nsplit))
+        work = torch.empty(floats, dtype=torch.float32, device=q.device) if floats else None
         st = torch.cuda.current_stream(q.device).cuda_stream
         N.check(N.lib().ptb_paged_attn_decode(q.data_ptr(), q.stride(0), out.data_ptr(), B, H, Hk, D, lens.data_ptr(),
                                               page_table.data_ptr(), page_table.stride(0), k_pages.shape[0], k_pages.data_ptr(),
