@@ -294,6 +294,155 @@ __global__ void __launch_bounds__(256) colsum2_kernel(const float* __restrict__ 
     }
 }
 
+// partial[CTA row][c] = sum over that CTA's rows of x[row][c]: 256 columns and a run of rows per CTA, a thread eight columns of every eighth row, four
+// rows in flight.  The gradient of a bias: bound by reading x once (16384 x 1536 bf16: 50 MB).
+template <typename T>
+__global__ void __launch_bounds__(256) colsum_rows_kernel(const T* __restrict__ x, long long rows, int N, long long ld, int per, float* __restrict__ partial) {
+    __shared__ float sm[8][264];
+    const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
+    const int c = blockIdx.x * 256 + cx * 8;
+    const long long r0 = (long long)blockIdx.y * per, r1 = min(r0 + per, rows);
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (c < N) {
+#pragma unroll 4
+        for (long long r = r0 + ry; r < r1; r += 8) {
+            Vec8<T> v;
+            float f[8];
+            v.load(x + r * ld + c);
+            v.get(f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] += f[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[ry][cx * 8 + j] = acc[j];
+    __syncthreads();
+    const int col = blockIdx.x * 256 + threadIdx.x;
+    if (col < N) {
+        float t = 0.f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) t += sm[r][threadIdx.x];
+        partial[(size_t)blockIdx.y * N + col] = t;
+    }
+}
+
+// ------------------------------------------------------------------------------------------ LayerNorm
+// A warp per row, the row in registers between the mean, the sum of squared deviations and the result.
+template <typename T, int MAXI>
+__global__ void __launch_bounds__(256) layernorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
+                                                            float* __restrict__ mean_out, float* __restrict__ rstd_out, long long rows, int H, float eps) {
+    const long long row = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31, nv = H / 8;
+    if (row >= rows) return;
+    float v[MAXI][8];
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < MAXI; ++k) {
+        const int i = k * 32 + lane;
+        if (i < nv) {
+            Vec8<T> t;
+            t.load(x + row * H + (size_t)i * 8);
+            t.get(v[k]);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) s += v[k][j];
+        }
+    }
+    const float mean = warp_sum(s) / (float)H;
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < MAXI; ++k)
+        if (k * 32 + lane < nv) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { v[k][j] -= mean; ss += v[k][j] * v[k][j]; }
+        }
+    const float rs = rsqrtf(warp_sum(ss) / (float)H + eps);
+    if (lane == 0) { mean_out[row] = mean; rstd_out[row] = rs; }
+#pragma unroll
+    for (int k = 0; k < MAXI; ++k) {
+        const int i = k * 32 + lane;
+        if (i < nv) {
+            Vec8<T> a, b, o;
+            float wf[8], bf[8], of[8];
+            a.load(w + (size_t)i * 8); b.load(bias + (size_t)i * 8);
+            a.get(wf); b.get(bf);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) of[j] = v[k][j] * rs * wf[j] + bf[j];
+            o.set(of);
+            o.store(y + row * H + (size_t)i * 8);
+        }
+    }
+}
+
+// dx, and per CTA the sums of dy * xhat and dy over its rows: dwb_partial [CTA][2][H].
+template <typename T, int MAXI>
+__global__ void __launch_bounds__(256) layernorm_bwd_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ dy, const float* __restrict__ mean_in,
+                                                            const float* __restrict__ rstd_in, T* __restrict__ dx, float* __restrict__ dwb_partial, long long rows, int H) {
+    __shared__ float sm[8][264];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nv = H / 8;
+    float dw[MAXI][8], db[MAXI][8];
+#pragma unroll
+    for (int k = 0; k < MAXI; ++k)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { dw[k][j] = 0.f; db[k][j] = 0.f; }
+    for (long long row = (long long)blockIdx.x * 8 + warp; row < rows; row += (long long)gridDim.x * 8) {
+        const float mean = mean_in[row], rs = rstd_in[row];
+        Vec8<T> xv[MAXI], gv[MAXI];
+#pragma unroll
+        for (int k = 0; k < MAXI; ++k) {
+            const int i = k * 32 + lane;
+            if (i < nv) { xv[k].load(x + row * H + (size_t)i * 8); gv[k].load(dy + row * H + (size_t)i * 8); }
+        }
+        float a = 0.f, c = 0.f;                       // sums of dy w and of dy w xhat
+#pragma unroll
+        for (int k = 0; k < MAXI; ++k) {
+            const int i = k * 32 + lane;
+            if (i < nv) {
+                Vec8<T> wv;
+                float xf[8], gf[8], wf[8];
+                wv.load(w + (size_t)i * 8);
+                xv[k].get(xf); gv[k].get(gf); wv.get(wf);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const float xh = (xf[j] - mean) * rs, gw = gf[j] * wf[j];
+                    a += gw; c += gw * xh;
+                    dw[k][j] += gf[j] * xh; db[k][j] += gf[j];
+                }
+            }
+        }
+        a = warp_sum(a) / (float)H;
+        c = warp_sum(c) / (float)H;
+#pragma unroll
+        for (int k = 0; k < MAXI; ++k) {
+            const int i = k * 32 + lane;
+            if (i < nv) {
+                Vec8<T> wv, o;
+                float xf[8], gf[8], wf[8], of[8];
+                wv.load(w + (size_t)i * 8);
+                xv[k].get(xf); gv[k].get(gf); wv.get(wf);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) of[j] = rs * (gf[j] * wf[j] - a - (xf[j] - mean) * rs * c);
+                o.set(of);
+                o.store(dx + row * H + (size_t)i * 8);
+            }
+        }
+    }
+    for (int part = 0; part < 2; ++part)
+#pragma unroll
+        for (int k = 0; k < MAXI; ++k) {
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) sm[warp][lane * 8 + j] = part ? db[k][j] : dw[k][j];
+            __syncthreads();
+            const int col = k * 256 + threadIdx.x;
+            if (col < H) {
+                float t = 0.f;
+#pragma unroll
+                for (int r = 0; r < 8; ++r) t += sm[r][threadIdx.x];
+                dwb_partial[((size_t)blockIdx.x * 2 + part) * H + col] = t;
+            }
+        }
+}
+
 // ------------------------------------------------------------------------------------------ rotary embedding
 // x: [B, T, heads, D] (contiguous), cos/sin: [T, D/2] fp32.  sign = +1 forward, -1 backward (the transpose).
 template <typename T>
@@ -578,6 +727,54 @@ PTB_API int ptb_rmsnorm_bwd(const void* x, const void* w, const void* dy, const 
     if (H % 8 || rms_threads(H) > 1024) { ptb_set_error("rmsnorm: hidden size %d not supported", H); return -1; }
     if (rows == 0) return 0;
     PTB_DISPATCH_T(bf16, launch_rmsnorm_bwd<T>(x, w, dy, rstd, dx, dw, dw_partial, n_ctas, rows, H, dresid, st));
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+// out[c] = sum over rows of x [rows, ld] (N columns, a multiple of eight, as are ld and the base in elements): fp32 sums, rounded once.  partial: n_parts * N floats.
+PTB_API int ptb_colsum(const void* x, long long rows, int N, long long ld, float* partial, int n_parts, void* out, int bf16, cudaStream_t st) {
+    if (N % 8 || ld % 8 || ((uintptr_t)x & 15) || n_parts < 1) { ptb_set_error("column sum: %d columns, pitch %lld not supported", N, ld); return -1; }
+    if (N <= 0) return 0;
+    const int per = (int)((rows + n_parts - 1) / n_parts);
+    const dim3 grid((N + 255) / 256, n_parts);
+    PTB_DISPATCH_T(bf16, (colsum_rows_kernel<T><<<grid, 256, 0, st>>>((const T*)x, rows, N, ld, per, partial),
+                          colsum2_kernel<T><<<(N + 31) / 32, 256, 0, st>>>(partial, n_parts, N, (T*)out)));
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+template <typename T>
+static void launch_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows, int H, float eps, cudaStream_t st) {
+    const unsigned grid = (unsigned)((rows + 7) / 8);
+    auto go = [&](auto kern) { kern<<<grid, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)b, (T*)y, mean, rstd, rows, H, eps); };
+    if (H <= 512) go(layernorm_fwd_kernel<T, 2>);
+    else go(layernorm_fwd_kernel<T, 4>);
+}
+template <typename T>
+static void launch_layernorm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd, void* dx, void* dwb, float* partial, int n_ctas,
+                                 long long rows, int H, cudaStream_t st) {
+    auto go = [&](auto kern) { kern<<<n_ctas, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, mean, rstd, (T*)dx, partial, rows, H); };
+    if (H <= 512) go(layernorm_bwd_kernel<T, 2>);
+    else go(layernorm_bwd_kernel<T, 4>);
+    colsum2_kernel<T><<<(2 * H + 31) / 32, 256, 0, st>>>(partial, n_ctas, 2 * H, (T*)dwb);
+}
+
+// LayerNorm over the last H of [rows, H] (H a multiple of eight up to 1024); mean, rstd fp32 [rows].
+PTB_API int ptb_layernorm_fwd(const void* x, const void* w, const void* b, void* y, float* mean, float* rstd, long long rows, int H, float eps, int bf16, cudaStream_t st) {
+    if (H % 8 || H > 1024 || H <= 0) { ptb_set_error("layernorm: size %d not supported", H); return -1; }
+    if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)b | (uintptr_t)y) & 15) { ptb_set_error("layernorm: needs 16-byte aligned tensors"); return -1; }
+    if (rows == 0) return 0;
+    PTB_DISPATCH_T(bf16, launch_layernorm_fwd<T>(x, w, b, y, mean, rstd, rows, H, eps, st));
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+// Its gradients: dx [rows, H], dwb [2, H] (of w, then of b); partial: n_ctas * 2 * H floats.
+PTB_API int ptb_layernorm_bwd(const void* x, const void* w, const void* dy, const float* mean, const float* rstd, void* dx, void* dwb, float* partial, int n_ctas,
+                              long long rows, int H, int bf16, cudaStream_t st) {
+    if (H % 8 || H > 1024 || H <= 0 || n_ctas < 1) { ptb_set_error("layernorm: size %d not supported", H); return -1; }
+    if (((uintptr_t)x | (uintptr_t)w | (uintptr_t)dy | (uintptr_t)dx) & 15) { ptb_set_error("layernorm: needs 16-byte aligned tensors"); return -1; }
+    PTB_DISPATCH_T(bf16, launch_layernorm_bwd<T>(x, w, dy, mean, rstd, dx, dwb, partial, n_ctas, rows, H, st));
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }

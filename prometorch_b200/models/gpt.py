@@ -9,7 +9,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..nn.fused import FusedCrossEntropyLoss, FusedLinear
+from ..nn.fused import FusedCrossEntropyLoss, FusedLayerNorm, FusedLinear
 from ..ops.attention import flash_attention
 
 
@@ -26,7 +26,7 @@ class GPTConfig:
 class GPTBlock(nn.Module):
     def __init__(self, c: GPTConfig):
         super().__init__()
-        self.ln1, self.ln2 = nn.LayerNorm(c.n_embd), nn.LayerNorm(c.n_embd)
+        self.ln1, self.ln2 = FusedLayerNorm(c.n_embd), FusedLayerNorm(c.n_embd)
         self.qkv = FusedLinear(c.n_embd, 3 * c.n_embd)
         self.proj = FusedLinear(c.n_embd, c.n_embd)
         self.fc = FusedLinear(c.n_embd, 4 * c.n_embd)
@@ -49,7 +49,7 @@ class CharGPT(nn.Module):
         self.wte = nn.Embedding(c.vocab_size, c.n_embd)
         self.wpe = nn.Embedding(c.block_size, c.n_embd)
         self.blocks = nn.ModuleList(GPTBlock(c) for _ in range(c.n_layer))
-        self.ln_f = nn.LayerNorm(c.n_embd)
+        self.ln_f = FusedLayerNorm(c.n_embd)
         self.loss_fn = FusedCrossEntropyLoss()
         self.apply(self._init)
 

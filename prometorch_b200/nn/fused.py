@@ -34,6 +34,15 @@ class FusedRMSNorm(nn.Module):
         return f"{self.weight.numel()}, eps={self.eps}"
 
 
+class FusedLayerNorm(nn.LayerNorm):
+    """``nn.LayerNorm`` whose bf16 CUDA path over one dimension is a kernel of its own, forward and backward."""
+
+    def forward(self, x):
+        if len(self.normalized_shape) == 1 and x.shape[-1] == self.normalized_shape[0] and K.layer_norm_ok(x, self.weight, self.bias):
+            return K.layer_norm(x, self.weight, self.bias, self.eps)
+        return super().forward(x)
+
+
 class FusedSwiGLU(nn.Module):
     """Gated MLP: ``down(act(gate(x)) * up(x))`` with gate and up stored as one ``[2*I, H]`` weight so a
     single GEMM produces both halves and one kernel applies the activation."""

@@ -30,7 +30,10 @@ def _decls(L):
     L.ptb_xent.argtypes = [vp, vp, vp, vp, vp, ll, ci, ll, cf, ll, ci, vp]
     L.ptb_xent_mean.argtypes = [vp, vp, vp, vp, ll, ci, ll, vp, ll, ci, vp]
     L.ptb_scale_unless_one.argtypes = [vp, ll, vp, ci, vp]
-    for n in ("ptb_rmsnorm_fwd", "ptb_rmsnorm_bwd", "ptb_rope", "ptb_gated_act_fwd", "ptb_gated_act_bwd", "ptb_xent", "ptb_xent_mean", "ptb_scale_unless_one"):
+    L.ptb_colsum.argtypes = [vp, ll, ci, ll, vp, ci, vp, ci, vp]
+    L.ptb_layernorm_fwd.argtypes = [vp, vp, vp, vp, vp, vp, ll, ci, cf, ci, vp]
+    L.ptb_layernorm_bwd.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, ci, ll, ci, ci, vp]
+    for n in ("ptb_colsum", "ptb_layernorm_fwd", "ptb_layernorm_bwd", "ptb_rmsnorm_fwd", "ptb_rmsnorm_bwd", "ptb_rope", "ptb_gated_act_fwd", "ptb_gated_act_bwd", "ptb_xent", "ptb_xent_mean", "ptb_scale_unless_one"):
         getattr(L, n).restype = ci
 
 
@@ -111,6 +114,64 @@ def add_rms_norm(x: torch.Tensor, resid: torch.Tensor, weight: torch.Tensor, eps
         h = x + resid
         return _rms_ref(h, weight, eps), h
     return _RMSNorm.apply(x, weight, eps, resid)
+
+
+# ----------------------------------------------------------------------------- LayerNorm, column sums
+def layer_norm_ok(x: torch.Tensor, w: Optional[torch.Tensor], b: Optional[torch.Tensor]) -> bool:
+    """bf16 on a GPU over up to 1024 features, scale and shift of the same type (other inputs keep torch's op, which differentiates further)."""
+    return (x.is_cuda and w is not None and b is not None and x.dtype == w.dtype == b.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0
+            and 0 < x.shape[-1] <= 1024 and tuple(w.shape) == tuple(b.shape) == (x.shape[-1],) and not torch.is_autocast_enabled("cuda"))
+
+
+def _aligned(t: torch.Tensor) -> torch.Tensor:
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
+class _LayerNorm(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, w, b, eps):
+        H = x.shape[-1]
+        x2, w, b = _aligned(x).view(-1, H), _aligned(w), _aligned(b)
+        y = torch.empty_like(x2)
+        mean, rstd = (torch.empty(x2.shape[0], dtype=torch.float32, device=x.device) for _ in range(2))
+        N.check(N.lib().ptb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), x2.shape[0], H, eps, _is_bf16(x2),
+                                          _stream(x)), "layernorm_fwd")
+        ctx.save_for_backward(x2, w, mean, rstd)
+        return y.view(x.shape)
+
+    @staticmethod
+    def backward(ctx, dy):
+        x2, w, mean, rstd = ctx.saved_tensors
+        rows, H = x2.shape
+        g = _aligned(dy).view(-1, H)
+        dx = torch.empty_like(x2)
+        n_ctas = max(1, min((rows + 7) // 8, _sms(x2.device) * 2))
+        dwb = torch.empty(2, H, dtype=w.dtype, device=w.device)
+        part = torch.empty(n_ctas * 2 * H, dtype=torch.float32, device=w.device)
+        N.check(N.lib().ptb_layernorm_bwd(x2.data_ptr(), w.data_ptr(), g.data_ptr(), mean.data_ptr(), rstd.data_ptr(), dx.data_ptr(), dwb.data_ptr(), part.data_ptr(),
+                                          n_ctas, rows, H, _is_bf16(x2), _stream(x2)), "layernorm_bwd")
+        return dx.view(dy.shape), dwb[0], dwb[1], None
+
+
+def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: float = 1e-5) -> torch.Tensor:
+    """``(x - mean) * rsqrt(var + eps) * weight + bias`` over the last dimension."""
+    if layer_norm_ok(x, weight, bias):
+        return _LayerNorm.apply(x, weight, bias, eps)
+    return F.layer_norm(x, x.shape[-1:], weight, bias, eps)
+
+
+def column_sum(x: torch.Tensor) -> torch.Tensor:
+    """Sum over the rows of ``x [rows, N]`` in fp32, in the type of ``x`` (a bias's gradient)."""
+    rows, n = x.shape
+    if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and rows and n and n % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+            and x.stride(0) >= n and x.data_ptr() % 16 == 0):
+        return x.float().sum(0).to(x.dtype)
+    parts = min(128, (rows + 63) // 64, max(1, 592 // ((n + 255) // 256)))
+    part = torch.empty(parts * n, dtype=torch.float32, device=x.device)
+    out = torch.empty(n, dtype=x.dtype, device=x.device)
+    N.check(N.lib().ptb_colsum(x.data_ptr(), rows, n, x.stride(0), part.data_ptr(), parts, out.data_ptr(), _is_bf16(x), _stream(x)), "colsum")
+    return out
 
 
 # ----------------------------------------------------------------------------- RoPE

@@ -136,7 +136,8 @@ class _Linear(torch.autograd.Function):
         if ctx.needs_input_grad[1]:
             dw = gemm_bf16(dy2, x2, a_mn=True, b_mn=True)                 # dW[out,in] = dY^T X
         if ctx.has_bias and ctx.needs_input_grad[2]:
-            db = dy2.float().sum(0).to(dy.dtype)
+            from .fused_ops import column_sum
+            db = column_sum(dy2)
         return dx, dw, db
 
 

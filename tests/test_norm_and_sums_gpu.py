@@ -1,8 +1,39 @@
 """LayerNorm, column sums and the optimizer's wide accesses at the edges of their shapes, against 64 bits."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("rows,H", [(1, 8), (7, 264), (33, 384), (2500, 512), (9, 520), (300, 1024)])
+def test_layer_norm(rows, H):
+    from prometorch_b200.ops.fused_ops import layer_norm
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    x = (torch.randn(rows, H, device="cuda", generator=g) * 2 + 5).bfloat16().requires_grad_()
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16().requires_grad_()
+    b = torch.randn(H, device="cuda", generator=g).bfloat16().requires_grad_()
+    dy = torch.randn(rows, H, device="cuda", generator=g).bfloat16()
+    y = layer_norm(x, w, b)
+    got = torch.autograd.grad(y, (x, w, b), dy)
+    r = [t.detach().double().requires_grad_() for t in (x, w, b)]
+    ry = F.layer_norm(r[0], (H,), r[1], r[2])
+    want = torch.autograd.grad(ry, r, dy.double())
+    # one rounding to bf16 (2^-8 of a value); in fp32 the sums of a row (2^-23 of terms up to 12 in size, H of them) and of a column
+    assert bool(((y.double() - ry).abs() <= 2 ** -8 * ry.abs() + 1e-4).all())
+    for a, c in zip(got, want):
+        assert bool(((a.double() - c).abs() <= 2 ** -8 * c.abs() + 1e-4 * (1 + c.abs().max())).all())
+
+
+@pytest.mark.parametrize("rows,N", [(1, 8), (65, 264), (8193, 1152), (300, 2056)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("pitch", [0, 8])
+def test_column_sum(rows, N, dtype, pitch):
+    from prometorch_b200.ops.fused_ops import column_sum
+    x = torch.randn(rows, N + pitch, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).to(dtype)[:, :N]
+    want = x.double().sum(0)
+    eps = 2 ** -8 if dtype == torch.bfloat16 else 2 ** -22
+    assert bool(((column_sum(x).double() - want).abs() <= eps * want.abs() + 2 ** -20 * rows ** 0.5 * 4).all())
 
 
 @pytest.mark.parametrize("n,off", [(1, 0), (4095, 0), (4099, 0), (65539, 0), (70000, 1)])
