@@ -379,13 +379,17 @@ static int launch(const void* q, long long ldq, const void* k, long long ldk, co
 // walks the query blocks that see those keys (all query heads of the KV head's group).  The scores are held transposed, a
 // tensor-memory lane per key, so that P^T is the A operand of dV from tensor memory.  Per query block i, in the order of issue:
 //   dV_j += P^T dO_i     P^T = exp2(S^T c - lse_i) in bf16, written by the compute warps over S^T
-//   dP^T = V_j dO_i^T
+//   dP^T = V_j dO_i^T    head size 128: its columns are those of dQ_i-1, which is read out under dV
 //   S^T  = K_j Q_i+1^T   the next block's scores
-//   dK_j += dS^T Q_i     dS^T = P^T (dP^T - delta_i) scale in bf16, in shared memory
-//   dQ_i = dS K_j        lands in dP's columns (head size 128) or its own (64)
-// so the exponentials of block i+1 run under dK and dQ of block i, dS under the next scores, and dQ's read-out under the next dV.
-// With all five products of a block in one chain behind its exponentials the tensor pipe idled more than half of the time
-// (2 x 4001 queries, 32 heads over 8, size 128, causal: 1.70 ms; now 0.95 ms, 690 TFLOP/s; 4 x 2048, 32 heads over 4, size 64: 0.73 -> 0.48 ms).
+//   dP^T = V_j dO_i+1^T  head size 64, where dQ has columns of its own: the next block's, too
+//   dQ_i = dS K_j        dS^T = P^T (dP^T - delta_i) scale in bf16, in shared memory
+//   dK_j += dS^T Q_i
+// so the exponentials of block i+1 run under dQ and dK of block i, and dS under the next scores.  CTAs start with the key blocks that most
+// queries see, over all heads: with one head's blocks after another the last head's longest one started near the end.
+// Measured (2 x 4001 queries, 32 heads over 8, size 128, causal; 4 x 2048, 32 over 4, size 64): all five products of a block in one chain behind its
+// exponentials 1.70 and 0.73 ms; in this order by heads 0.95 and 0.41 ms (size 64 with dP behind its own exponentials 0.43; size 128 with the next
+// dP ahead, behind dQ's read-out: 1.06), long CTAs first 0.84 and 0.34 ms.  Bound by the compute warps' latency (issue slots 22 to 29 % used,
+// tensor pipe 25 to 35 %).
 // Every tile lives in shared memory in ONE layout, [64-column chunk][row][128 B, 128-byte swizzle], which the
 // descriptors read as a K-major operand (rows = M or N) or as an MN-major operand (rows = K): Q_i is the B operand
 // of S^T and of dK, dO_i that of dP^T and of dV, K_j the A operand of S^T and the B operand of dQ, and dS^T
@@ -460,10 +464,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     uint64_t* dp_full = bars + 10;       // dP^T is in TMEM
     uint64_t* p_ready = bars + 11;       // P^T is in TMEM (8 arrivals)
     uint64_t* ds_ready = bars + 12;      // dS^T is in shared memory (8 arrivals)
-    uint64_t* dq_full = bars + 13;       // dK updated, dQ_i in TMEM
+    uint64_t* dq_full = bars + 13;       // dQ_i is in TMEM
     uint64_t* dq_read = bars + 14;       // dQ_i has been read back (4 arrivals)
     uint64_t* all_done = bars + 15;      // dK and dV are complete
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
+    uint64_t* ds_empty = bars + 16;      // the MMAs that read dS^T have completed
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
     if (smem_u32(smem) & 1023) {         // the swizzled tiles need it, and there is no room to align by hand
@@ -471,7 +476,9 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         return;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int jb = blockIdx.x, hk = blockIdx.y / P.gsplit, part = blockIdx.y % P.gsplit, b = blockIdx.z;
+    // early key blocks (with a causal mask those that most queries see) first, over all heads and sequences: the last CTAs to start are short
+    const int per_jb = P.Hk * P.gsplit * P.B, jb = (int)blockIdx.x / per_jb, unit = (int)blockIdx.x % per_jb;
+    const int hk = unit % P.Hk, part = unit / P.Hk % P.gsplit, b = unit / (P.Hk * P.gsplit);
     const int group = (P.H / P.Hk) / P.gsplit;          // query heads this CTA walks
     const int head0 = hk * (P.H / P.Hk) + part * group;
     const int key0 = jb * 128;
@@ -485,7 +492,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
         mbar_init(kv_full, 1);
         for (int st = 0; st < 2; ++st) { mbar_init(&q_full[st], 1); mbar_init(&q_empty[st], 1); mbar_init(&do_full[st], 1); mbar_init(&do_empty[st], 1); }
         mbar_init(s_full, 1); mbar_init(dp_full, 1); mbar_init(p_ready, 8); mbar_init(ds_ready, 8);
-        mbar_init(dq_full, 1); mbar_init(dq_read, 4); mbar_init(all_done, 1);
+        mbar_init(dq_full, 1); mbar_init(dq_read, 4); mbar_init(all_done, 1); mbar_init(ds_empty, 1);
         *abort_flag = 0;
         mbar_fence_init();
         prefetch_tmap(&tmQ); prefetch_tmap(&tmK); prefetch_tmap(&tmV); prefetch_tmap(&tmDO); prefetch_tmap(&tmDQ);
@@ -543,22 +550,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 umma_commit(s_full);
                 return true;
             };
-            bool ok = mbar_wait(kv_full, 0, P.status) && issue_s(0);
-            for (int it = 0; it < n_it && ok; ++it) {
-                const uint32_t aQ = smem_u32(sq + (it & 1) * S::TILE), aDO = smem_u32(sdo + (it % NDO) * S::TILE);
-                const uint32_t ph = (uint32_t)(it & 1), acc = it > 0 ? 1u : 0u;
-                ok = mbar_wait(&do_full[it % NDO], (uint32_t)((it / NDO) & 1), P.status) && mbar_wait(p_ready, ph, P.status);
-                if (!ok) break;
+            auto issue_dp = [&](int it) {
+                const int st = it % NDO;
+                const uint32_t aDO = smem_u32(sdo + st * S::TILE);
+                if (!mbar_wait(&do_full[st], (uint32_t)((it / NDO) & 1), P.status)) return false;
                 tc_fence_after();
-#pragma unroll
-                for (int kq = 0; kq < 8; ++kq)        // K dimension = the 128 queries, 16 per step: 2048 B further down each chunk of dO
-                    umma_bf16_ts(tmem_base + TM_DV, tmem_base + TM_S + (uint32_t)((kq >> 2) * 64 + (kq & 3) * 8), smem_desc(aDO + kq * 2048, 16384, 1024), idesc_k,
-                                 (kq > 0) ? 1u : acc);
-                if (TM_DQ == TM_DP && it > 0) {       // dQ_i-1 leaves these columns while dV runs
-                    ok = mbar_wait(dq_read, ph ^ 1, P.status);
-                    if (!ok) break;
-                    tc_fence_after();
-                }
 #pragma unroll
                 for (int c = 0; c < D / 64; ++c)
 #pragma unroll
@@ -566,21 +562,46 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                         umma_bf16(tmem_base + TM_DP, smem_desc(aV + c * 16384 + k * 32, 16, 1024), smem_desc(aDO + c * 16384 + k * 32, 16, 1024), idesc_t,
                                   (c > 0 || k > 0) ? 1u : 0u);
                 umma_commit(dp_full);
-                umma_commit(&do_empty[it % NDO]);
-                if (it + 1 < n_it) ok = issue_s(it + 1);
-                if (ok) ok = mbar_wait(ds_ready, ph, P.status);
-                if (ok && TM_DQ != TM_DP && it > 0) ok = mbar_wait(dq_read, ph ^ 1, P.status);
+                return true;
+            };
+            constexpr bool AHEAD = D == 64;               // dP^T of the next block before this block is done
+            bool ok = mbar_wait(kv_full, 0, P.status) && issue_s(0) && (!AHEAD || issue_dp(0));
+            for (int it = 0; it < n_it && ok; ++it) {
+                const uint32_t aQ = smem_u32(sq + (it & 1) * S::TILE), aDO = smem_u32(sdo + (it % NDO) * S::TILE);
+                const uint32_t ph = (uint32_t)(it & 1), acc = it > 0 ? 1u : 0u;
+                ok = mbar_wait(p_ready, ph, P.status);
                 if (!ok) break;
                 tc_fence_after();
+#pragma unroll
+                for (int kq = 0; kq < 8; ++kq)        // K dimension = the 128 queries, 16 per step: 2048 B further down each chunk of dO
+                    umma_bf16_ts(tmem_base + TM_DV, tmem_base + TM_S + (uint32_t)((kq >> 2) * 64 + (kq & 3) * 8), smem_desc(aDO + kq * 2048, 16384, 1024), idesc_k,
+                                 (kq > 0) ? 1u : acc);
+                if (!AHEAD) {                         // dQ_i-1 leaves these columns while dV runs
+                    if (it > 0) ok = mbar_wait(dq_read, ph ^ 1, P.status);
+                    if (ok) ok = issue_dp(it);
+                    if (!ok) break;
+                }
+                umma_commit(&do_empty[it % NDO]);
+                if (it + 1 < n_it) ok = issue_s(it + 1);
+                if (ok) ok = mbar_wait(ds_ready, ph, P.status);          // dS^T is written, and dP^T has been read
+                if (!ok) break;
+                tc_fence_after();
+                if (AHEAD) {
+                    if (it + 1 < n_it) ok = issue_dp(it + 1);
+                    if (ok && it > 0) ok = mbar_wait(dq_read, ph ^ 1, P.status);
+                    if (!ok) break;
+                    tc_fence_after();
+                }
+#pragma unroll
+                for (int kk = 0; kk < 8; ++kk)        // K dimension = the 128 keys
+                    umma_bf16(tmem_base + TM_DQ, smem_desc(aDS + kk * 2048, 16384, 1024), smem_desc(aK + kk * 2048, 16384, 1024), idesc_q, kk > 0 ? 1u : 0u);
+                umma_commit(dq_full);
 #pragma unroll
                 for (int kq = 0; kq < 8; ++kq)
                     umma_bf16(tmem_base + TM_DK, smem_desc(aDS + (kq >> 2) * 16384 + (kq & 3) * 32, 16, 1024), smem_desc(aQ + kq * 2048, 16384, 1024), idesc_k,
                               (kq > 0) ? 1u : acc);
                 umma_commit(&q_empty[it & 1]);
-#pragma unroll
-                for (int kk = 0; kk < 8; ++kk)        // K dimension = the 128 keys
-                    umma_bf16(tmem_base + TM_DQ, smem_desc(aDS + kk * 2048, 16384, 1024), smem_desc(aK + kk * 2048, 16384, 1024), idesc_q, kk > 0 ? 1u : 0u);
-                umma_commit(dq_full);
+                umma_commit(ds_empty);
             }
             umma_commit(all_done);
             if (!ok) *abort_flag = 1;
@@ -690,6 +711,7 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             if (ok && !*abort_flag) ok = mbar_wait(dp_full, (uint32_t)(it & 1), P.status);
             else ok = false;
             tc_fence_after();
+            if (it > 0 && ok) ok = mbar_wait(ds_empty, (uint32_t)((it - 1) & 1), P.status);
             uint8_t* drow = sds + hf * 16384 + row * 128;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -780,8 +802,10 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
     p.lse = lse; p.delta = delta; p.dk = (__nv_bfloat16*)dk; p.dv = (__nv_bfloat16*)dv;
     p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
     p.scale = scale; p.scale_log2 = scale * 1.4426950408889634f; p.status = status; p.gsplit = gsplit;
-    dim3 grid((Tk + 127) / 128, Hk * gsplit, B);
-    bwd_kernel<D><<<grid, BWD_THREADS, SmB<D>::TOTAL, st>>>(mq, mk, mv, mdo, mdq, p);
+    const long long ctas = (long long)((Tk + 127) / 128) * Hk * gsplit * B;
+    if (ctas > 0x7fffffffLL) { ptb_set_error("flash attention: %lld tiles", ctas); return -1; }
+    if (ctas == 0) return 0;
+    bwd_kernel<D><<<(unsigned)ctas, BWD_THREADS, SmB<D>::TOTAL, st>>>(mq, mk, mv, mdo, mdq, p);
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
 }
