@@ -275,6 +275,104 @@ __global__ void __launch_bounds__(256) rmsnorm_bwd_warp_kernel(const T* __restri
     }
 }
 
+// The same for wide bf16 rows: 128 threads a row, two rows a CTA.  x and dy of a row stay in registers (packed) from the reduction to the result, and the
+// next row's are requested before the reduction, so a row costs its bytes once; with a warp per row, which reads them twice and
+// waits for each row alone, 8192 x 2048 took 50 us and 4096 x 4096 100 us.
+template <int V>
+__global__ void __launch_bounds__(256) rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy,
+                                                               const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_partial,
+                                                               long long rows, int H, const __nv_bfloat16* __restrict__ dresid) {
+    using T = __nv_bfloat16;
+    __shared__ float red[2][2][4];
+    __shared__ float4 other[V * 2 * 128];
+    const int grp = threadIdx.x >> 7, t = threadIdx.x & 127, nv = H / 8;
+    const long long step = (long long)gridDim.x * 2;
+    Vec8<T> wv[V], nx[V], ng[V];
+    float dw[V][8], rs_n = 0.f;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        if (k * 128 + t < nv) wv[k].load(w + (size_t)(k * 128 + t) * 8);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
+    }
+    auto fetch = [&](long long row) {
+        if (row >= rows) return;
+        rs_n = rstd[row];
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int i = k * 128 + t;
+            if (i < nv) { nx[k].load(x + row * H + (size_t)i * 8); ng[k].load(dy + row * H + (size_t)i * 8); }
+        }
+    };
+    long long row = (long long)blockIdx.x * 2 + grp;
+    fetch(row);
+    for (int par = 0; row < rows; row += step, par ^= 1) {
+        Vec8<T> cx[V], cg[V], cr[V];
+        const float rs = rs_n;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            cx[k] = nx[k]; cg[k] = ng[k];
+            const int i = k * 128 + t;
+            if (dresid && i < nv) cr[k].load(dresid + row * H + (size_t)i * 8);
+        }
+        fetch(row + step);
+        float dot = 0.f;
+#pragma unroll
+        for (int k = 0; k < V; ++k)
+            if (k * 128 + t < nv) {
+                float xf[8], gf[8], wf[8];
+                cx[k].get(xf); cg[k].get(gf); wv[k].get(wf);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) dot += gf[j] * wf[j] * xf[j];
+            }
+        dot = warp_sum(dot);
+        if ((t & 31) == 0) red[grp][par][t >> 5] = dot;
+        asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory");
+        dot = (red[grp][par][0] + red[grp][par][1]) + (red[grp][par][2] + red[grp][par][3]);
+        const float c = dot * rs * rs * rs / (float)H;
+#pragma unroll
+        for (int k = 0; k < V; ++k) {
+            const int i = k * 128 + t;
+            if (i < nv) {
+                float xf[8], gf[8], wf[8], of[8];
+                cx[k].get(xf); cg[k].get(gf); wv[k].get(wf);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    of[j] = rs * gf[j] * wf[j] - c * xf[j];
+                    dw[k][j] += gf[j] * xf[j] * rs;
+                }
+                if (dresid) {
+                    float rf[8];
+                    cr[k].get(rf);
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) of[j] += rf[j];
+                }
+                Vec8<T> o;
+                o.set(of);
+                o.store(dx + row * H + (size_t)i * 8);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+        if (grp) {
+            other[(2 * k) * 128 + t] = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
+            other[(2 * k + 1) * 128 + t] = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
+        }
+    __syncthreads();
+    if (grp) return;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+        const int i = k * 128 + t;
+        if (i < nv) {
+            const float4 a = other[(2 * k) * 128 + t], b = other[(2 * k + 1) * 128 + t];
+            float4* p = reinterpret_cast<float4*>(dw_partial + (size_t)blockIdx.x * H + (size_t)i * 8);
+            p[0] = make_float4(dw[k][0] + a.x, dw[k][1] + a.y, dw[k][2] + a.z, dw[k][3] + a.w);
+            p[1] = make_float4(dw[k][4] + b.x, dw[k][5] + b.y, dw[k][6] + b.z, dw[k][7] + b.w);
+        }
+    }
+}
+
 // out[c] = sum_p partial[p][c]: 32 columns per CTA, eight row groups summed in parallel, then combined.
 template <typename T>
 __global__ void __launch_bounds__(256) colsum2_kernel(const float* __restrict__ partial, int P, int H, T* __restrict__ out) {
@@ -711,7 +809,11 @@ PTB_API int ptb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, 
 template <typename T>
 static void launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, void* dw, float* dw_partial,
                                int n_ctas, long long rows, int H, const void* dresid, cudaStream_t st) {
-    if (H <= 2048) {
+    using B = __nv_bfloat16;
+    auto wide = [&](auto kern) { kern<<<n_ctas, 256, 0, st>>>((const B*)x, (const B*)w, (const B*)dy, rstd, (B*)dx, dw_partial, rows, H, (const B*)dresid); };
+    if (sizeof(T) == 2 && H > 1024 && H <= 2048) wide(rmsnorm_bwd_wide_kernel<2>);
+    else if (sizeof(T) == 2 && H > 2048 && H <= 4096) wide(rmsnorm_bwd_wide_kernel<4>);
+    else if (H <= 2048) {
         rmsnorm_bwd_warp_kernel<T, 8><<<n_ctas, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, (const T*)dresid);
     } else if (H <= 4096) {
         rmsnorm_bwd_warp_kernel<T, 16><<<n_ctas, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, (const T*)dresid);

@@ -60,3 +60,30 @@ def test_optimizer_wide_and_narrow(n, off):
         w = w * (1 - 1e-3) - 1e-2 * (m / (1 - 0.9 ** t)) / ((v / (1 - 0.95 ** t)).sqrt() + 1e-8)
     # fp32 arithmetic of a few operations on values up to 5: 2^-20
     assert float((p.double() - w).abs().max()) < 5 * 2 ** -20 and torch.equal(low, p.detach().bfloat16())
+
+
+@pytest.mark.parametrize("rows,H", [(1, 1032), (3, 2048), (700, 2040), (1, 2056), (601, 4096), (5, 4088)])
+@pytest.mark.parametrize("resid", [False, True])
+def test_rms_norm_backward_wide_rows(rows, H, resid):
+    """Two and four 16-byte pieces a thread, the last ones partly past the row; one row (half of a CTA idle) and more rows than CTAs take at once."""
+    from prometorch_b200.ops.fused_ops import add_rms_norm, rms_norm
+    g = torch.Generator(device="cuda").manual_seed(rows + H)
+    x = torch.randn(rows, H, device="cuda", generator=g).bfloat16().requires_grad_()
+    r = torch.randn(rows, H, device="cuda", generator=g).bfloat16().requires_grad_()
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16().requires_grad_()
+    dy, dh = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    if resid:
+        y, h = add_rms_norm(x, r, w)
+        got = torch.autograd.grad((y, h), (x, w), (dy, dh))
+        v = h.detach().double().requires_grad_()
+    else:
+        got = torch.autograd.grad(rms_norm(x, w), (x, w), dy)
+        v = x.detach().double().requires_grad_()
+    wd = w.detach().double().requires_grad_()
+    ref = v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-6) * wd
+    want = list(torch.autograd.grad(ref, (v, wd), dy.double()))
+    if resid:
+        want[0] = want[0] + dh.double()
+    # one rounding to bf16 over fp32 sums of up to 4096 terms (2^-23 each)
+    for a, b in zip(got, want):
+        assert bool(((a.double() - b).abs() <= 2 ** -8 * b.abs() + 1e-4 * (1 + b.abs().max())).all())
