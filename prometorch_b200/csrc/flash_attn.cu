@@ -151,31 +151,34 @@ __global__ void __launch_bounds__(THREADS) fwd_kernel(const __grid_constant__ Fw
     }
 }
 
-// delta[b,h,t] = sum_d dO * O
+// delta[b,h,t] = sum_d dO * O.  D / 8 lanes a row, 16 bytes of each operand a lane: a pass at the bytes it moves (4 bytes a lane and one
+// row a warp took 67 us over 2 x 4001 x 32 rows of 128, 262 MB with the cleared dQ).
 template <int D>
-__global__ void delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
-                             long long rows, int H, int Tq, float* __restrict__ dq_zero = nullptr) {
-    const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;     // one warp per (b, t, h) row
-    const int lane = threadIdx.x & 31;
-    if (w >= rows) return;
-    const __nv_bfloat16* op = o + w * D;
-    const __nv_bfloat16* dp = dout + w * D;
-    if (dq_zero) {          // the fp32 dQ accumulator has the same [B, Tq, H, D] rows: clear this one on the way
-        for (int i = lane * 4; i < D; i += 128) *reinterpret_cast<float4*>(dq_zero + w * D + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
+__global__ void __launch_bounds__(256) delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ dout, float* __restrict__ delta,
+                                                    long long rows, int H, int Tq, float* __restrict__ dq_zero = nullptr) {
+    constexpr int LANES = D / 8;
+    const long long w = ((long long)blockIdx.x * 256 + threadIdx.x) / LANES;        // row (b, t, h)
+    const int l = threadIdx.x % LANES;
     float s = 0.f;
-    for (int i = lane * 2; i < D; i += 64) {
-        const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(op + i));
-        const float2 b2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(dp + i));
-        s += a.x * b2.x + a.y * b2.y;
+    if (w < rows) {
+        const uint4 a = *reinterpret_cast<const uint4*>(o + w * D + l * 8), b = *reinterpret_cast<const uint4*>(dout + w * D + l * 8);
+        if (dq_zero) {          // the fp32 dQ accumulator has the same [B, Tq, H, D] rows: clear this one on the way
+            float4* z = reinterpret_cast<float4*>(dq_zero + w * D + l * 8);
+            z[0] = z[1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        const __nv_bfloat162 *a2 = reinterpret_cast<const __nv_bfloat162*>(&a), *b2 = reinterpret_cast<const __nv_bfloat162*>(&b);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 x = __bfloat1622float2(a2[i]), y = __bfloat1622float2(b2[i]);
+            s += x.x * y.x + x.y * y.y;
+        }
     }
-    s = warp_sum(s);
-    if (lane == 0) {
+#pragma unroll
+    for (int m = LANES / 2; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if (w < rows && l == 0) {
         const long long bt = w / H;
         const int h = (int)(w % H);
-        const long long b = bt / Tq;
-        const int tq = (int)(bt % Tq);
-        delta[(b * H + h) * Tq + tq] = s;
+        delta[(bt / Tq * H + h) * Tq + bt % Tq] = s;
     }
 }
 
@@ -366,7 +369,7 @@ PTB_API int ptb_flash_attn_fwd(const void* q, const void* k, const void* v, void
 template <int D>
 static int run_bwd(const BwdParams& p, const void* o, cudaStream_t st) {
     const long long rows = (long long)p.B * p.Tq * p.H;
-    delta_kernel<D><<<(unsigned)((rows * 32 + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, p.dout, const_cast<float*>(p.delta), rows, p.H, p.Tq);
+    delta_kernel<D><<<(unsigned)((rows * (D / 8) + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, p.dout, const_cast<float*>(p.delta), rows, p.H, p.Tq);
     constexpr int smem = 4 * BC * D * 2 + BC * BR * 2 + 2 * BR * 4;
     static bool attr = false;
     if (!attr) { PTB_CUDA_OK(cudaFuncSetAttribute(bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)); attr = true; }
@@ -381,7 +384,7 @@ static int run_bwd(const BwdParams& p, const void* o, cudaStream_t st) {
 PTB_API int ptb_flash_attn_delta(const void* o, const void* dout, float* delta, int B, int Tq, int H, int D, float* dq_zero, cudaStream_t st) {
     const long long rows = (long long)B * Tq * H;
     if (rows == 0) return 0;
-    const unsigned grid = (unsigned)((rows * 32 + 255) / 256);
+    const unsigned grid = (unsigned)((rows * (D / 8) + 255) / 256);
     if (D == 64) delta_kernel<64><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, H, Tq, dq_zero);
     else if (D == 128) delta_kernel<128><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, H, Tq, dq_zero);
     else { ptb_set_error("flash attention: head_dim %d not supported", D); return -1; }
