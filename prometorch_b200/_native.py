@@ -33,6 +33,17 @@ class LayerDesc(C.Structure):
                 ("window", C.c_int), ("pad", C.c_int), ("post_attn_norm", C.c_void_p), ("post_ffn_norm", C.c_void_p)]
 
 
+class PromptLayer(C.Structure):
+    _fields_ = [("w", C.c_void_p * 7), ("qtype", C.c_int * 7), ("pad", C.c_int), ("ffn_norm", C.c_void_p), ("next_norm", C.c_void_p),
+                ("q_norm", C.c_void_p), ("k_norm", C.c_void_p), ("k_cache", C.c_void_p), ("v_cache", C.c_void_p)]
+
+
+class PromptRun(C.Structure):
+    _fields_ = [(n, C.c_int) for n in ("T", "H", "heads", "kv_heads", "D", "I", "S", "layout", "gelu", "add_one", "neox", "n_sm")] + \
+               [("eps", C.c_float), ("scale", C.c_float), ("cos", C.c_void_p), ("sin", C.c_void_p), ("offsets", C.c_void_p), ("x", C.c_void_p * 2)] + \
+               [(n, C.c_void_p) for n in ("h", "qkv", "att", "o", "gate_up", "act", "weights", "work")] + [("work_floats", C.c_longlong), ("status", C.c_void_p)]
+
+
 class ModelDesc(C.Structure):
     _fields_ = [("n_layers", C.c_int), ("hidden", C.c_int), ("n_heads", C.c_int), ("n_kv_heads", C.c_int),
                 ("head_dim", C.c_int), ("inter", C.c_int), ("vocab", C.c_int), ("max_seq", C.c_int),
@@ -93,6 +104,10 @@ def _declare(L: C.CDLL):
     L.ptb_dequant_weights.restype = ci
     L.ptb_prompt_heads.argtypes = [vp, ci, ci, ci, ci, vp, vp, ci, C.c_float, vp, vp, ci, ci, vp, vp, ci, vp]
     L.ptb_prompt_heads.restype = ci
+    L.ptb_prompt_work_floats.argtypes = [C.POINTER(PromptRun)]
+    L.ptb_prompt_work_floats.restype = C.c_longlong
+    L.ptb_prompt_layers.argtypes = [C.POINTER(PromptLayer), ci, C.POINTER(PromptRun), vp]
+    L.ptb_prompt_layers.restype = ci
     L.ptb_dequant_rows.argtypes = [vp, ci, ci, ci, vp, ci, cf, ci, vp, vp, vp]
     L.ptb_dequant_rows.restype = ci
 

@@ -194,3 +194,36 @@ typedef struct PtbStreamStep {
     int top, e_rows, taps, slots, pos_stride, req_stride, n, m, W, streams, bf16;
     float eps;
 } PtbStreamStep;
+
+// One layer of a quantised model as its prompt pass reads it: matrices in a GEMV streaming layout, bf16 norms (ready to multiply), fp16 caches.
+typedef struct PtbPromptLayer {
+    const void* w[7];       // q, k, v, o, gate, up, down
+    int qtype[7];
+    int pad;
+    const void* ffn_norm;   // bf16 [H]: norm of the stream after the attention
+    const void* next_norm;  // bf16 [H]: the next layer's first norm, or the output norm; null in a last layer that ends at its cache
+    const float* q_norm;    // fp32 [D] or null
+    const float* k_norm;
+    void* k_cache;          // fp16 [Hk, S, D]
+    void* v_cache;
+} PtbPromptLayer;
+
+// A prompt of T tokens from position 0 and the buffers it runs in (all 16-byte aligned, bf16 unless said otherwise).
+typedef struct PtbPromptRun {
+    int T, H, heads, kv_heads, D, I, S, layout, gelu, add_one, neox, n_sm;
+    float eps, scale;
+    const float* cos;       // fp32 [S, D/2]
+    const float* sin;
+    const int* offsets;     // device {0, T}
+    void* x[2];             // [T, H]: the stream enters in x[0]
+    void* h;                // [T, H]: normed rows; the first norm enters, the last one leaves
+    void* qkv;              // [T, (heads + 2 kv_heads) D]
+    void* att;              // [T, heads D]
+    void* o;                // [T, H]
+    void* gate_up;          // [T, 2 I]
+    void* act;              // [T, I]
+    void* weights;          // room for the largest group of matrices
+    float* work;            // ptb_prompt_work_floats floats
+    long long work_floats;
+    int* status;
+} PtbPromptRun;

@@ -492,6 +492,37 @@ class GGUFModel:
         shape = (self.local_kv_heads, self.max_seq, self.cfg.head_dim)
         return self._wrap(k.value, n, torch.float16).view(shape), self._wrap(v.value, n, torch.float16).view(shape)
 
+    def _prompt_layers(self, x, h, T: int, offs_dev, nw, to_the_end: bool, st: int) -> torch.Tensor:
+        """The layers over a prompt from position 0, launched by the native library (csrc/prompt_layers.cu): no biases, norms only before the
+        sublayers, one GPU.  ``x``: the stream, ``h``: its first norm.  Returns the rows after the output norm (meaningless unless ``to_the_end``)."""
+        from ..ops.gemm import _sms, _status
+        cfg, dev, n = self.cfg, self.device, len(self.layers)
+        H, D, hq, hkv, I = cfg.hidden_size, cfg.head_dim, self.local_heads, self.local_kv_heads, self.local_inter
+        layers = (N.PromptLayer * n)()
+        for i, (dst, L) in enumerate(zip(layers, self.layers)):
+            for j, name in enumerate(("q", "k", "v", "o", "gate", "up", "down")):
+                dst.w[j], dst.qtype[j] = L[name].data.data_ptr(), L[name].qtype
+            dst.ffn_norm, dst.q_norm, dst.k_norm = N.ptr(nw(L, "ffn_norm")), N.ptr(L["q_norm"]), N.ptr(L["k_norm"])
+            dst.next_norm = N.ptr(nw(self.layers[i + 1], "attn_norm")) if i + 1 < n else N.ptr(self._out_norm_bf16) if to_the_end else None
+            k, v = C.c_void_p(), C.c_void_p()
+            N.check(self._lib.ptb_engine_kv_cache(self._engine, i, C.byref(k), C.byref(v)), "kv_cache")
+            dst.k_cache, dst.v_cache = k.value, v.value
+        rows = max((hq + 2 * hkv) * D * H, H * hq * D, 2 * I * H)                   # elements of the largest group of matrices
+        if "prompt" not in self._dq_scratch:
+            self._dq_scratch["prompt"] = torch.empty(rows, dtype=torch.bfloat16, device=dev)
+        buf = lambda cols: torch.empty(T, cols, dtype=torch.bfloat16, device=dev)
+        x1, qkv, att, o, gu, act = buf(H), buf((hq + 2 * hkv) * D), buf(hq * D), buf(H), buf(2 * I), buf(I)
+        r = N.PromptRun(T=T, H=H, heads=hq, kv_heads=hkv, D=D, I=I, S=self.max_seq, layout=self.layout, gelu=int(bool(cfg.ffn_gelu)),
+                        add_one=int(bool(cfg.gemma_norm_add_one)), neox=int(bool(cfg.rope_neox)), n_sm=_sms(dev), eps=cfg.rms_norm_eps, scale=D ** -0.5,
+                        cos=self.cos.data_ptr(), sin=self.sin.data_ptr(), offsets=offs_dev.data_ptr(), h=h.data_ptr(), qkv=qkv.data_ptr(), att=att.data_ptr(),
+                        o=o.data_ptr(), gate_up=gu.data_ptr(), act=act.data_ptr(), weights=self._dq_scratch["prompt"].data_ptr(), status=_status(x.device).data_ptr())
+        r.x[0], r.x[1] = x.data_ptr(), x1.data_ptr()
+        r.work_floats = self._lib.ptb_prompt_work_floats(C.byref(r))
+        work = torch.empty(max(1, r.work_floats), dtype=torch.float32, device=dev)
+        r.work = work.data_ptr()
+        N.check(self._lib.ptb_prompt_layers(layers, n, C.byref(r), st), "prompt_layers")
+        return h
+
     @torch.no_grad()
     def prefill(self, tokens: Sequence[int], pos0: int = 0, return_logits: bool = False):
         """Run ``tokens`` at positions ``pos0 ..`` through the model in ONE batched pass that fills the KV cache:
@@ -504,7 +535,8 @@ class GGUFModel:
         if not self.supports_prefill:
             raise NotImplementedError("batched prefill: no sliding window, head size 64 or 128")
         from ..ops import fused_ops as K
-        from ..ops.attention import flash_attention, flash_attention_varlen
+        from ..ops import gemm as G
+        from ..ops.attention import _use_tcgen05, flash_attention, flash_attention_varlen
         from ..ops.gemm import linear, linear_add_rms_norm, linear_swiglu
         cfg, dev = self.cfg, self.device
         T = len(tokens)
@@ -560,7 +592,12 @@ class GGUFModel:
         offs = [0, T]
         offs_dev = torch.tensor(offs, dtype=torch.int32, device=dev)
         h = K.rms_norm(x, nw(self.layers[0], "attn_norm"), eps)
-        for i, L in enumerate(self.layers):
+        plain = pos0 == 0 and self.tp_world == 1 and G._SPLITK and _use_tcgen05() and all(
+            L["post_attn_norm"] is None and L["post_ffn_norm"] is None and all(L[n].bias is None for n in ("q", "k", "v", "o", "gate", "up", "down"))
+            for L in self.layers)
+        if plain:
+            h = self._prompt_layers(x, h, T, offs_dev, nw, return_logits, st)
+        for i, L in enumerate(() if plain else self.layers):
             last = i + 1 == len(self.layers)
             qkv = linear(h, self._dequant(L["q"], L["k"], L["v"]), bias_of(L, "qkv_bias", ("q", "k", "v")))
             kc, vc = self._kv_views(i)
