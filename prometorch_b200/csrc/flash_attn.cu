@@ -366,8 +366,15 @@ PTB_API int ptb_flash_attn_fwd(const void* q, const void* k, const void* v, void
     return D == 64 ? run_fwd<64>(p, st) : run_fwd<128>(p, st);
 }
 
+// What the delta pass reads and clears in 16-byte pieces.
+static int delta_operands_ok(const void* o, const void* dout, const float* dq_zero) {
+    if (((uintptr_t)o | (uintptr_t)dout | (uintptr_t)dq_zero) & 15) { ptb_set_error("flash attention: outputs and their gradients need a 16-byte aligned base"); return 0; }
+    return 1;
+}
+
 template <int D>
 static int run_bwd(const BwdParams& p, const void* o, cudaStream_t st) {
+    if (!delta_operands_ok(o, p.dout, nullptr)) return -1;
     const long long rows = (long long)p.B * p.Tq * p.H;
     delta_kernel<D><<<(unsigned)((rows * (D / 8) + 255) / 256), 256, 0, st>>>((const __nv_bfloat16*)o, p.dout, const_cast<float*>(p.delta), rows, p.H, p.Tq);
     constexpr int smem = 4 * BC * D * 2 + BC * BR * 2 + 2 * BR * 4;
@@ -384,6 +391,7 @@ static int run_bwd(const BwdParams& p, const void* o, cudaStream_t st) {
 PTB_API int ptb_flash_attn_delta(const void* o, const void* dout, float* delta, int B, int Tq, int H, int D, float* dq_zero, cudaStream_t st) {
     const long long rows = (long long)B * Tq * H;
     if (rows == 0) return 0;
+    if (!delta_operands_ok(o, dout, dq_zero)) return -1;
     const unsigned grid = (unsigned)((rows * (D / 8) + 255) / 256);
     if (D == 64) delta_kernel<64><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, H, Tq, dq_zero);
     else if (D == 128) delta_kernel<128><<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)dout, delta, rows, H, Tq, dq_zero);

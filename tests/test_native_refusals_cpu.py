@@ -1,0 +1,28 @@
+"""Operands that a kernel of the native library could not read are refused on the host, before any launch."""
+import ctypes as C
+
+import pytest
+
+BASE = 1 << 20          # an aligned address; nothing is read from it
+
+
+def _lib():
+    from prometorch_b200 import _native as N
+    import prometorch_b200.ops.attention  # noqa: F401  (its prototypes)
+    return N.lib()
+
+
+def _refused(rc):
+    return rc == -1 and _lib().ptb_last_error().decode()
+
+
+@pytest.mark.parametrize("off_o,off_do,off_dq", [(4, 0, 0), (0, 2, 0), (0, 8, 0), (0, 0, 4)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_flash_attention_delta_needs_aligned_rows(off_o, off_do, off_dq, D):
+    L = _lib()
+    vp = C.c_void_p
+    L.ptb_flash_attn_delta.argtypes = [vp, vp, vp, C.c_int, C.c_int, C.c_int, C.c_int, vp, vp]
+    assert "16-byte aligned" in _refused(L.ptb_flash_attn_delta(BASE + off_o, BASE + off_do, BASE, 1, 8, 2, D, BASE + off_dq, None))
+    if not off_dq:      # the backward that takes no buffer to clear
+        assert "16-byte aligned" in _refused(L.ptb_flash_attn_bwd(BASE, BASE, BASE, BASE + off_o, BASE + off_do, BASE, BASE, BASE, BASE, BASE, 0, 1, 8, 8, 2, 2, D, 1,
+                                                                  1.0, 0, None))
