@@ -138,11 +138,13 @@ def flash_attention_varlen(q, k, v, offs, offs_dev: Optional[torch.Tensor] = Non
     tensor on the device.  Returns ``[n, H, D]``.  Inference on a GPU is one launch; otherwise it is :func:`flash_attention` per sequence."""
     n, H, D = q.shape
     Hk = k.shape[1]
+    if tuple(k.shape) != (n, Hk, D) or v.shape[:2] != k.shape[:2] or not offs or offs[0] != 0 or offs[-1] != n or any(b < a for a, b in zip(offs, offs[1:])):
+        raise ValueError(f"packed attention: sequences {list(offs)[:4]}... over q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
     scale = scale if scale is not None else 1.0 / math.sqrt(D)
     rows_ok = all(t.stride(2) == 1 and t.stride(1) == D and t.stride(0) % 8 == 0 and t.stride(0) >= t.shape[1] * D and t.data_ptr() % 16 == 0 for t in (q, k, v))
     same = all(t.dtype == torch.bfloat16 and t.is_cuda for t in (q, k, v))
     grad = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, v))
-    if n and same and rows_ok and not grad and D in (64, 128) and H % Hk == 0 and offs_dev is not None and _use_tcgen05():
+    if n and same and rows_ok and not grad and D == v.shape[2] and D in (64, 128) and H % Hk == 0 and offs_dev is not None and _use_tcgen05():
         from .gemm import _status
         out = torch.empty(n, H, D, dtype=q.dtype, device=q.device)
         st = torch.cuda.current_stream(q.device).cuda_stream

@@ -149,6 +149,15 @@ def test_attention_reference_path(B, Tq, Tk, H, Hk, D, off, causal):
         assert torch.allclose(o1 * w1 + o2 * w2, o, atol=1e-5)
 
 
+@pytest.mark.parametrize("bad", [dict(offs=[0, 3]), dict(offs=[0, 9]), dict(offs=[1, 8]), dict(offs=[0, 5, 4, 8]), dict(offs=[]), dict(k=7), dict(v=7), dict(vh=1)])
+def test_packed_attention_refuses_what_does_not_fit(bad):
+    """A kernel that took the rows of k and v from q would read past their end."""
+    import prometorch_b200.ops.attention as A
+    q, k, v = torch.randn(8, 4, 64), torch.randn(bad.get("k", 8), 2, 64), torch.randn(bad.get("v", 8), bad.get("vh", 2), 64)
+    with pytest.raises(ValueError, match="packed attention"):
+        A.flash_attention_varlen(q, k, v, bad.get("offs", [0, 3, 8]))
+
+
 @pytest.mark.parametrize("bias", [True, False])
 @pytest.mark.parametrize("m,k,n", [(1, 1, 1), (3, 16, 8), (2 * 5, 64, 24), (33, 130, 7)], ids=str)
 def test_linear_family(m, k, n, bias):
