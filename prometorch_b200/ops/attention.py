@@ -135,7 +135,8 @@ def flash_attention(q, k, v, causal: bool = True, q_offset: int = 0, scale: Opti
 def flash_attention_varlen(q, k, v, offs, offs_dev: Optional[torch.Tensor] = None, scale: Optional[float] = None):
     """Causal attention of packed sequences: sequence i is the rows ``offs[i]:offs[i + 1]`` of ``q [n, H, D]`` and ``k``, ``v [n, Hk, D]``
     (heads next to one another; rows may be further apart, as in columns of a packed projection).  ``offs`` is a list, ``offs_dev`` the same as an int32
-    tensor on the device.  Returns ``[n, H, D]``.  Inference on a GPU is one launch; otherwise it is :func:`flash_attention` per sequence."""
+    tensor on the device.  Returns ``[n, H, D]``.  Inference on a GPU is one launch; otherwise it is :func:`flash_attention`, one call for
+    neighbouring sequences of one length."""
     n, H, D = q.shape
     Hk = k.shape[1]
     if tuple(k.shape) != (n, Hk, D) or v.shape[:2] != k.shape[:2] or not offs or offs[0] != 0 or offs[-1] != n or any(b < a for a, b in zip(offs, offs[1:])):
@@ -152,4 +153,13 @@ def flash_attention_varlen(q, k, v, offs, offs_dev: Optional[torch.Tensor] = Non
                                                   len(offs) - 1, max(b - a for a, b in zip(offs, offs[1:])), n, H, Hk, D, 1, scale,
                                                   _status(q.device).data_ptr(), st), "flash_attn_varlen")
         return out
-    return torch.cat([flash_attention(q[a:b][None], k[a:b][None], v[a:b][None], causal=True, scale=scale)[0] for a, b in zip(offs, offs[1:])])
+    out, i = [], 0
+    while i + 1 < len(offs):
+        a, m = offs[i], offs[i + 1] - offs[i]
+        j = i + 1
+        while j + 1 < len(offs) and offs[j + 1] - offs[j] == m:
+            j += 1
+        if m:
+            out.append(flash_attention(*(t[a:offs[j]].reshape(j - i, m, *t.shape[1:]) for t in (q, k, v)), causal=True, scale=scale).reshape(offs[j] - a, H, -1))
+        i = j
+    return torch.cat(out) if out else q.new_empty(0, H, v.shape[2])

@@ -149,6 +149,21 @@ def test_attention_reference_path(B, Tq, Tk, H, Hk, D, off, causal):
         assert torch.allclose(o1 * w1 + o2 * w2, o, atol=1e-5)
 
 
+def test_packed_attention_shares_calls(monkeypatch):
+    """Without the one-launch kernel, neighbouring sequences of one length are one call, as are those of length zero none."""
+    import prometorch_b200.ops.attention as A
+    lens = [5, 5, 3, 0, 7, 7, 7, 5]
+    offs = [sum(lens[:i]) for i in range(len(lens) + 1)]
+    g = torch.Generator().manual_seed(1)
+    x = torch.randn(offs[-1], 4 + 2 * 2, 16, generator=g, dtype=torch.float64)
+    q, k, v = x[:, :4], x[:, 4:6], x[:, 6:]
+    want = torch.cat([A.attention_reference(q[None, a:b], k[None, a:b], v[None, a:b], True)[0][0] for a, b in zip(offs, offs[1:]) if b > a])
+    calls, inner = [], A.flash_attention
+    monkeypatch.setattr(A, "flash_attention", lambda q, *r, **kw: calls.append(tuple(q.shape[:2])) or inner(q, *r, **kw))
+    torch.testing.assert_close(A.flash_attention_varlen(q, k, v, offs), want, rtol=1e-5, atol=1e-6)
+    assert calls == [(2, 5), (1, 3), (3, 7), (1, 5)]
+
+
 @pytest.mark.parametrize("bad", [dict(offs=[0, 3]), dict(offs=[0, 9]), dict(offs=[1, 8]), dict(offs=[0, 5, 4, 8]), dict(offs=[]), dict(k=7), dict(v=7), dict(vh=1)])
 def test_packed_attention_refuses_what_does_not_fit(bad):
     """A kernel that took the rows of k and v from q would read past their end."""
