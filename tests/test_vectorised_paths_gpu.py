@@ -66,6 +66,21 @@ def test_cross_entropy_gradient_of_the_mean(V, rows, dtype, up):
     assert float((x.grad.double() - r.grad).abs().max()) <= 2 * eps * abs(up) / max(1, int((t >= 0).sum()))
 
 
+@pytest.mark.parametrize("V", [512, 33])
+@pytest.mark.parametrize("up", [1.0, 0.25])
+@pytest.mark.parametrize("inplace", [False, True])
+def test_cross_entropy_second_backward_is_refused(V, up, inplace):
+    """The gradient is scaled in place, so a second pass over the same graph would scale it twice."""
+    from prometorch_b200.ops.fused_ops import cross_entropy
+    x = torch.randn(9, V, device="cuda", generator=torch.Generator(device="cuda").manual_seed(V)).bfloat16().requires_grad_()
+    loss = cross_entropy(x * 1.0, torch.arange(9, device="cuda"), inplace_grad=inplace) * up
+    loss.backward(retain_graph=True)
+    first = x.grad.clone()
+    with pytest.raises(RuntimeError, match="inplace"):
+        loss.backward()
+    assert torch.equal(x.grad, first)
+
+
 @pytest.mark.parametrize("kinds", [("Q4_K", "Q4_K", "Q6_K"), ("Q6_K", "Q4_K"), ("Q4_K", "Q8_0", "Q6_K"), ("Q6_K",)])
 @pytest.mark.parametrize("rows", [(40, 8, 24), (16, 1, 7)])
 @pytest.mark.parametrize("layout", [0, 1])
