@@ -19,6 +19,7 @@
 #include "gemm_sm100.cuh"
 
 int ptb_make_tmap_bf16(CUtensorMap* map, const void* base, long long inner, long long outer, long long ld, int box_inner, int box_outer);
+int ptb_make_tmap_bf16_3d(CUtensorMap* map, const void* base, long long n0, long long n1, long long n2, int b0, int b1, int b2);
 int ptb_make_tmap_f32_3d(CUtensorMap* map, const void* base, long long n0, long long n1, long long n2, int b0, int b1);
 
 namespace ptb {
@@ -433,6 +434,11 @@ struct SmB {
     static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)), "l"(map),
+                 "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
 __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1),
                  "r"(c2)
@@ -516,8 +522,8 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
             bool ok = true;
             mbar_expect_tx(kv_full, 2 * S::TILE);
             for (int c = 0; c < D / 64; ++c) {
-                tma_load_2d(sk + c * 16384, &tmK, hk * D + c * 64, b * P.Tk + key0, kv_full);
-                tma_load_2d(sv + c * 16384, &tmV, hk * D + c * 64, b * P.Tk + key0, kv_full);
+                tma_load_3d(sk + c * 16384, &tmK, hk * D + c * 64, key0, b, kv_full);
+                tma_load_3d(sv + c * 16384, &tmV, hk * D + c * 64, key0, b, kv_full);
             }
             for (int it = 0; it < n_it && ok; ++it) {
                 const int h = head0 + it / per_head, i = i_start + it % per_head;
@@ -525,11 +531,11 @@ bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
                 if (it >= 2) ok = mbar_wait(&q_empty[qs], (uint32_t)(((it >> 1) - 1) & 1), P.status);
                 if (!ok) break;
                 mbar_expect_tx(&q_full[qs], S::TILE);
-                for (int c = 0; c < D / 64; ++c) tma_load_2d(sq + qs * S::TILE + c * 16384, &tmQ, h * D + c * 64, b * P.Tq + i * 128, &q_full[qs]);
+                for (int c = 0; c < D / 64; ++c) tma_load_3d(sq + qs * S::TILE + c * 16384, &tmQ, h * D + c * 64, i * 128, b, &q_full[qs]);
                 if (it >= NDO) ok = mbar_wait(&do_empty[ds], (uint32_t)(((it / NDO) - 1) & 1), P.status);
                 if (!ok) break;
                 mbar_expect_tx(&do_full[ds], S::TILE);
-                for (int c = 0; c < D / 64; ++c) tma_load_2d(sdo + ds * S::TILE + c * 16384, &tmDO, h * D + c * 64, b * P.Tq + i * 128, &do_full[ds]);
+                for (int c = 0; c < D / 64; ++c) tma_load_3d(sdo + ds * S::TILE + c * 16384, &tmDO, h * D + c * 64, i * 128, b, &do_full[ds]);
             }
             if (!ok) *abort_flag = 1;
         } else if (warp == 9 && lane == 0 && n_it > 0) {
@@ -790,10 +796,12 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
                       cudaStream_t st) {
     CUtensorMap mq, mk, mv, mdo, mdq;
     if (ptb_make_tmap_f32_3d(&mdq, dq, (long long)H * D, Tq, B, 32, 128)) return -1;
-    if (ptb_make_tmap_bf16(&mq, q, (long long)H * D, (long long)B * Tq, (long long)H * D, 64, 128)) return -1;
-    if (ptb_make_tmap_bf16(&mdo, dout, (long long)H * D, (long long)B * Tq, (long long)H * D, 64, 128)) return -1;
-    if (ptb_make_tmap_bf16(&mk, k, (long long)Hk * D, (long long)B * Tk, (long long)Hk * D, 64, 128)) return -1;
-    if (ptb_make_tmap_bf16(&mv, v, (long long)Hk * D, (long long)B * Tk, (long long)Hk * D, 64, 128)) return -1;
+    // Rows past an entry's end arrive as zeros.  As rows of one [B T] matrix they were the next entry's: their weights are zero, but zero times
+    // what is not finite is not, and one entry's infinities reached the gradients of the entry before it.
+    if (ptb_make_tmap_bf16_3d(&mq, q, (long long)H * D, Tq, B, 64, 128, 1)) return -1;
+    if (ptb_make_tmap_bf16_3d(&mdo, dout, (long long)H * D, Tq, B, 64, 128, 1)) return -1;
+    if (ptb_make_tmap_bf16_3d(&mk, k, (long long)Hk * D, Tk, B, 64, 128, 1)) return -1;
+    if (ptb_make_tmap_bf16_3d(&mv, v, (long long)Hk * D, Tk, B, 64, 128, 1)) return -1;
     static bool attr = false;
     if (!attr) {
         PTB_CUDA_OK(cudaFuncSetAttribute(bwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmB<D>::TOTAL));

@@ -72,3 +72,22 @@ def test_backward_tiles(B, Tq, Tk, H, Hk, D, causal, off):
     for a, b in zip(got, want):
         # P, dS and the results rounded to bf16 once each, delta from an output rounded to bf16; a single key has no gradient but rounding
         assert float((a.double() - b).norm()) < 6e-3 * float(b.norm()) + 2 ** -9 * float(do.norm())
+
+
+@pytest.mark.parametrize("Tq,Tk,causal", [(129, 129, True), (130, 70, False), (1, 257, False)])
+@pytest.mark.parametrize("D", [64, 128])
+def test_entries_of_a_batch_stay_apart(Tq, Tk, causal, D):
+    """Ragged last blocks lie over the next entry's rows: what is not finite there reaches neither outputs nor gradients of the entry before."""
+    from prometorch_b200.ops.attention import flash_attention
+    g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
+    one = [torch.randn(1, t, h, D, device="cuda", generator=g).bfloat16() for t, h in ((Tq, 4), (Tk, 2), (Tk, 2), (Tq, 4))]
+
+    def run(x):
+        q, k, v = (t.clone().requires_grad_() for t in x[:3])
+        o = flash_attention(q, k, v, causal=causal)
+        return [o.detach(), *torch.autograd.grad(o, (q, k, v), x[3])]
+    want = run(one)
+    for bad in (float("inf"), float("nan")):
+        got = run([torch.cat([t, torch.full_like(t, bad)]) for t in one])
+        for a, b in zip(got, want):             # the order in which key blocks are added to dQ is free
+            assert bool(torch.isfinite(a[0]).all()) and _rel(a[0], b[0].double()) < 1e-3
