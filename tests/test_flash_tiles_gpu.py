@@ -91,3 +91,26 @@ def test_entries_of_a_batch_stay_apart(Tq, Tk, causal, D):
         got = run([torch.cat([t, torch.full_like(t, bad)]) for t in one])
         for a, b in zip(got, want):             # the order in which key blocks are added to dQ is free
             assert bool(torch.isfinite(a[0]).all()) and _rel(a[0], b[0].double()) < 1e-3
+
+
+@pytest.mark.parametrize("peak", [1.0, 3.0])
+@pytest.mark.parametrize("D", [64, 128])
+def test_forward_error_is_that_of_exact_maxima(peak, D):
+    """Weights are rounded to bf16 under the running maximum of each block: no further from 64 bits than the same roundings in 64-bit arithmetic."""
+    from prometorch_b200.ops.attention import flash_attention
+    T, H, two = 1025, 2, 1.4426950408889634
+    g = torch.Generator(device="cuda").manual_seed(D)
+    q, k, v = ((torch.randn(T, H, D, device="cuda", generator=g) * s).bfloat16() for s in (peak, 1, 1))
+    o = flash_attention(q[None], k[None], v[None], causal=True)[0]
+    s = torch.einsum("qhd,khd->hqk", q.double(), k.double()) * D ** -0.5 * two
+    s = s.masked_fill(torch.ones(T, T, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    vd = v.double().transpose(0, 1)
+    want = torch.softmax(s / two, -1) @ vd
+    m, total, acc = s[..., :1], 0.0, 0.0
+    for j in range(0, T, 128):
+        grown = torch.maximum(m, s[..., j:j + 128].amax(-1, keepdim=True))
+        p = torch.exp2(s[..., j:j + 128] - grown)
+        alpha, m = torch.exp2(m - grown), grown
+        total, acc = total * alpha + p.sum(-1, keepdim=True), acc * alpha + p.bfloat16().double() @ vd[:, j:j + 128]
+    # what is left is the arithmetic in 32 bits, a hundredth of a bf16 rounding
+    assert _rel(o.transpose(0, 1), want) <= 1.01 * _rel((acc / total).bfloat16(), want)
