@@ -117,10 +117,16 @@ def add_rms_norm(x: torch.Tensor, resid: torch.Tensor, weight: torch.Tensor, eps
 
 
 # ----------------------------------------------------------------------------- LayerNorm, column sums
+def _transformed() -> bool:
+    """Whether a trace, a compilation, a function transform (vmap, grad, jvp) or forward-mode differentiation sees the ops that run: raw kernels are not for it."""
+    return (torch.jit.is_tracing() or torch.compiler.is_compiling() or torch._C._functorch.peek_interpreter_stack() is not None
+            or torch.autograd.forward_ad._current_level >= 0)
+
+
 def layer_norm_ok(x: torch.Tensor, w: Optional[torch.Tensor], b: Optional[torch.Tensor]) -> bool:
-    """bf16 on a GPU over up to 1024 features, scale and shift of the same type (other inputs keep torch's op, which differentiates further)."""
+    """bf16 on a GPU over up to 1024 features, scale and shift of the same type, outside of autocast, traces and function transforms (the rest keeps torch's op)."""
     return (x.is_cuda and w is not None and b is not None and x.dtype == w.dtype == b.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0
-            and 0 < x.shape[-1] <= 1024 and tuple(w.shape) == tuple(b.shape) == (x.shape[-1],) and not torch.is_autocast_enabled("cuda"))
+            and 0 < x.shape[-1] <= 1024 and tuple(w.shape) == tuple(b.shape) == (x.shape[-1],) and not torch.is_autocast_enabled("cuda") and not _transformed())
 
 
 def _aligned(t: torch.Tensor) -> torch.Tensor:
@@ -132,18 +138,23 @@ class _LayerNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, b, eps):
         H = x.shape[-1]
-        x2, w, b = _aligned(x).view(-1, H), _aligned(w), _aligned(b)
+        x2, w2, b2 = _aligned(x).view(-1, H), _aligned(w), _aligned(b)
         y = torch.empty_like(x2)
         mean, rstd = (torch.empty(x2.shape[0], dtype=torch.float32, device=x.device) for _ in range(2))
-        N.check(N.lib().ptb_layernorm_fwd(x2.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), x2.shape[0], H, eps, _is_bf16(x2),
+        N.check(N.lib().ptb_layernorm_fwd(x2.data_ptr(), w2.data_ptr(), b2.data_ptr(), y.data_ptr(), mean.data_ptr(), rstd.data_ptr(), x2.shape[0], H, eps, _is_bf16(x2),
                                           _stream(x)), "layernorm_fwd")
-        ctx.save_for_backward(x2, w, mean, rstd)
+        ctx.save_for_backward(x, w, b, mean, rstd)
         return y.view(x.shape)
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w, mean, rstd = ctx.saved_tensors
-        rows, H = x2.shape
+        x, w, b, mean, rstd = ctx.saved_tensors
+        H = x.shape[-1]
+        if torch.is_grad_enabled():           # create_graph: torch's backward, which differentiates again
+            stat = (*x.shape[:-1], 1)
+            return (*torch.ops.aten.native_layer_norm_backward(dy, x, [H], mean.view(stat), rstd.view(stat), w, b, list(ctx.needs_input_grad[:3])), None)
+        x2, w = _aligned(x).view(-1, H), _aligned(w)
+        rows = x2.shape[0]
         g = _aligned(dy).view(-1, H)
         dx = torch.empty_like(x2)
         n_ctas = max(1, min((rows + 7) // 8, _sms(x2.device) * 2))
@@ -164,7 +175,7 @@ def layer_norm(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor, eps: f
 def column_sum(x: torch.Tensor) -> torch.Tensor:
     """Sum over the rows of ``x [rows, N]`` in fp32, in the type of ``x`` (a bias's gradient)."""
     rows, n = x.shape
-    if not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and rows and n and n % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
+    if (torch.is_grad_enabled() and x.requires_grad) or not (x.is_cuda and x.dtype in (torch.bfloat16, torch.float32) and rows and n and n % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0
             and x.stride(0) >= n and x.data_ptr() % 16 == 0):
         return x.float().sum(0).to(x.dtype)
     parts = min(128, (rows + 63) // 64, max(1, 592 // ((n + 255) // 256)))

@@ -25,6 +25,32 @@ def test_layer_norm(rows, H):
         assert bool(((a.double() - c).abs() <= 2 ** -8 * c.abs() + 1e-4 * (1 + c.abs().max())).all())
 
 
+def test_layer_norm_and_column_sum_differentiate_twice():
+    """Under ``create_graph`` and in function transforms the values are those of torch's op, derivatives of the gradients among them."""
+    from prometorch_b200.nn.fused import FusedLayerNorm
+    from prometorch_b200.ops.fused_ops import column_sum
+    g = torch.Generator(device="cuda").manual_seed(3)
+    x, dy, u = (torch.randn(5, 64, device="cuda", generator=g).bfloat16().requires_grad_() for _ in range(3))
+    m = FusedLayerNorm(64, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        m.weight.copy_(1 + 0.1 * torch.randn(64, device="cuda", generator=g))
+        m.bias.copy_(torch.randn(64, device="cuda", generator=g))
+    def second(x, dy, w, b):
+        dx, dw, db = torch.autograd.grad(F.layer_norm(x, (64,), w, b) if x.dtype == torch.float64 else m(x), (x, w, b), dy, create_graph=True)
+        return torch.autograd.grad((dx * u.to(dx.dtype)).sum() + (dw * dw).sum() + (db * db).sum(), (x, dy, w))
+    got = second(x, dy, m.weight, m.bias)
+    want = second(*(t.detach().double().requires_grad_() for t in (x, dy, m.weight, m.bias)))
+    for a, b in zip(got, want):              # a handful of roundings to bf16 (2^-9 each, relative to the largest terms)
+        assert float((a.double() - b).norm() / b.norm()) < 2e-2
+    c, = torch.autograd.grad(column_sum(dy).float().square().sum(), dy)
+    assert float((c.double() - 2 * dy.detach().double().sum(0)).norm() / c.double().norm()) < 1e-2
+    plain = F.layer_norm(x, (64,), m.weight, m.bias)
+    assert torch.allclose(torch.func.vmap(m)(x[:, None])[:, 0].float(), plain.float(), atol=2e-2)
+    _, jvp = torch.func.jvp(m, (x.detach(),), (u.detach(),))
+    _, ref = torch.func.jvp(lambda t: F.layer_norm(t, (64,), m.weight, m.bias), (x.detach(),), (u.detach(),))
+    assert torch.equal(jvp, ref)
+
+
 @pytest.mark.parametrize("rows,N", [(1, 8), (65, 264), (8193, 1152), (300, 2056)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("pitch", [0, 8])
