@@ -35,10 +35,15 @@ class FusedRMSNorm(nn.Module):
 
 
 class FusedLayerNorm(nn.LayerNorm):
-    """``nn.LayerNorm`` whose bf16 CUDA path over one dimension is a kernel of its own, forward and backward."""
+    """``nn.LayerNorm`` whose bf16 CUDA path over one dimension is a kernel of its own, forward and backward, for large inputs.
+
+    The kernel saves the GPU about 15 us per million values (16384 x 384: 132 us forward and backward with torch's op, 38 here; 4096 x 384: 48
+    and 26), but as a Python function it costs the host 46 us more than torch's op.  Up to ``LARGE`` values the host is what bounds a step
+    of the models that use it (four 384-wide layers, 16384 tokens: 5.5 ms of host work beside 4.8 of GPU work with torch's op)."""
+    LARGE = 1 << 23
 
     def forward(self, x):
-        if len(self.normalized_shape) == 1 and x.shape[-1] == self.normalized_shape[0] and K.layer_norm_ok(x, self.weight, self.bias):
+        if x.numel() >= self.LARGE and len(self.normalized_shape) == 1 and x.shape[-1] == self.normalized_shape[0] and K.layer_norm_ok(x, self.weight, self.bias):
             return K.layer_norm(x, self.weight, self.bias, self.eps)
         return super().forward(x)
 

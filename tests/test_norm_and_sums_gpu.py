@@ -25,6 +25,17 @@ def test_layer_norm(rows, H):
         assert bool(((a.double() - c).abs() <= 2 ** -8 * c.abs() + 1e-4 * (1 + c.abs().max())).all())
 
 
+def test_layer_norm_module_keeps_the_native_op_for_small_inputs():
+    """Below ``LARGE`` values the kernel costs the host more than it saves the GPU."""
+    from prometorch_b200.nn.fused import FusedLayerNorm
+    m = FusedLayerNorm(512, device="cuda", dtype=torch.bfloat16)
+    rows = FusedLayerNorm.LARGE // 512
+    small, large = (torch.randn(n, 512, device="cuda", dtype=torch.bfloat16, requires_grad=True) for n in (rows - 1, rows))
+    assert m(small).grad_fn.name() == "NativeLayerNormBackward0" and "_LayerNorm" in m(large).grad_fn.name()
+    ref = F.layer_norm(large.double(), (512,))
+    assert bool(((m(large).double() - ref).abs() <= 2 ** -8 * ref.abs() + 1e-4).all())          # one rounding to bf16 over fp32 sums
+
+
 def test_layer_norm_and_column_sum_differentiate_twice():
     """Under ``create_graph`` and in function transforms the values are those of torch's op, derivatives of the gradients among them."""
     from prometorch_b200.nn.fused import FusedLayerNorm
@@ -32,6 +43,7 @@ def test_layer_norm_and_column_sum_differentiate_twice():
     g = torch.Generator(device="cuda").manual_seed(3)
     x, dy, u = (torch.randn(5, 64, device="cuda", generator=g).bfloat16().requires_grad_() for _ in range(3))
     m = FusedLayerNorm(64, device="cuda", dtype=torch.bfloat16)
+    m.LARGE = 0
     with torch.no_grad():
         m.weight.copy_(1 + 0.1 * torch.randn(64, device="cuda", generator=g))
         m.bias.copy_(torch.randn(64, device="cuda", generator=g))
