@@ -630,6 +630,9 @@ PTB_API int ptb_gemm_bf16(const void* A, long long lda, int a_mn, const void* B,
 // Floats of workspace with which ptb_gemm_bf16_ws cuts the tiles of the last wave along K (0: it would not).
 PTB_API long long ptb_gemm_work_floats(int M, int N, int K, int n_sm) { return plan_pair(M, N, K, n_sm, true).work_floats; }
 
+// Whether a plain product of these sizes runs on pairs of SMs, with the workspace that ptb_gemm_work_floats asks for or without one.
+PTB_API int ptb_gemm_on_pairs(int M, int N, int K, int n_sm, int with_work) { return plan_pair(M, N, K, n_sm, with_work != 0).use; }
+
 // The same with a workspace of `work_floats` floats (16-byte aligned) for partial sums.
 PTB_API int ptb_gemm_bf16_ws(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C, long long ldc, int M, int N, int K,
                              const float* bias, int flags, float* work, long long work_floats, int* status, int n_sm, cudaStream_t st) {

@@ -25,6 +25,8 @@ def _decls(L):
     L.ptb_gemm_bf16.restype = ci
     L.ptb_gemm_work_floats.argtypes = [ci, ci, ci, ci]
     L.ptb_gemm_work_floats.restype = ll
+    L.ptb_gemm_on_pairs.argtypes = [ci, ci, ci, ci, ci]
+    L.ptb_gemm_on_pairs.restype = ci
     L.ptb_gemm_bf16_ws.argtypes = [vp, ll, ci, vp, ll, ci, vp, ll, ci, ci, ci, vp, ci, vp, ll, vp, ci, vp]
     L.ptb_gemm_bf16_ws.restype = ci
     if hasattr(L, "ptb_gemm_bf16_splitk"):
