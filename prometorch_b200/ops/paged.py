@@ -121,15 +121,19 @@ def qkv_rope_write(h: torch.Tensor, wqkv: torch.Tensor, H: int, Hk: int, D: int,
 
 
 def pick_splits(B: int, Hk: int, max_len: int, sms: int = 148) -> int:
-    """Splits of the page walk, each a CTA of eight warps and of at least a page; a power of two (the choice is a key of the engine's graph
-    cache, so it should change rarely).  Splits pay until every SM has a CTA, and beyond that only where each keeps a long walk: launching
-    and merging clusters costs more than idle SMs.  Measured, us: 1 request, 4 kv heads, 540 tokens: 12.0 (1 split), 6.2 (16); 32 requests, 4 heads of a
-    group of 4, 300 tokens: 8.4 (1), 9.2 (2), 25.3 (8), 1500 tokens: 36.7 (1), 29.6 (2), 45.9 (8); 8 requests, 32 heads, 1800 tokens: 42.3 (1), 49.6 (2)."""
+    """Splits of the page walk, each a CTA of eight warps (two to an SM) and of about half a page or more; a power of two (the choice is a key of the
+    engine's graph cache, so it should change rarely).  Splits pay until every SM has a CTA; up to two an SM where each keeps 512 tokens; and where
+    the CTAs do not fit the GPU at once and walk 4096 tokens or more, since a last wave of shorter ones wastes less.  Elsewhere launching and merging clusters costs
+    more than idle SMs.  Measured, us with a cold L2, splits in brackets:
+    1 request, 4 kv heads in groups of 4, 540 tokens: 20.5 (1), 12.4 (8), 12.3 (16); 8 kv heads, 129 tokens: 12.3 (1), 10.3 (4), 12.4 (16);
+    32 requests, 4 kv heads in groups of 4, 300 tokens: 16.5 (1), 22.6 (4); 1500 tokens: 47.0 (1), 38.9 (2), 43.0 (4);
+    24 requests, 32 kv heads, 8192 tokens (768 CTAs): 473 (1), 484 (2); 64 requests, 8 kv heads, 8192 (512): 426 (1), 351 (2); 16384, groups of 4: 1033 (1), 926 (2), 981 (4);
+    8 requests, 32 kv heads (256, which fit): 186 (1), 230 (2), 189 (4); 32768: 662 (1), 839 (2), 664 (4); 64 requests, 4 kv heads in groups of 4, 8192: 270 (1), 273 (2)."""
     pages = max(1, (max_len + PAGE - 1) // PAGE)
     n = 1
     while n < 16 and n < pages:
-        ctas, each = 2 * n * B * Hk, max_len // (2 * n)
-        if not (ctas <= sms or (ctas <= 2 * sms and each >= 512) or (ctas <= 8 * sms and each >= 4096)):
+        now, each = n * B * Hk, max_len // (2 * n)
+        if not (2 * now <= sms or (2 * now <= 2 * sms and each >= 512) or (2 * sms < now <= 4 * sms and each >= 4096)):
             break
         n *= 2
     return n

@@ -212,6 +212,7 @@ def test_paged_ops_reference_paths():
         ref = torch.einsum("hn,nhd->hd", torch.softmax(s, -1), v).reshape(-1)
         assert torch.allclose(out[b], ref, atol=1e-5)
     assert P.pick_splits(1, 8, 8192) == 16 and P.pick_splits(64, 8, 8192) == 2 and P.pick_splits(4, 4, 64) == 1
+    assert P.pick_splits(8, 32, 8192) == P.pick_splits(8, 32, 32768) == 1          # 256 CTAs fit at once: two splits each took 24 % longer
 
 
 def test_speculative_decoding_gives_the_same_greedy_tokens():
