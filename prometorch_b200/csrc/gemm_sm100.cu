@@ -161,12 +161,12 @@ struct SplitK { int splits; long long stride; int bn; int pdl; };      // splits
 // Whether a product runs on pairs of SMs, and how.  Times are in units of the pair kernel's k-block (256 x 256 x 64 on two SMs, about 0.33 us);
 // a 128 x 256 tile's k-block takes its one SM 1.3 of them and a 128 x 128 tile's 0.85 (measured over the products of the 2048- and
 // 4096-wide models, forward, both gradients: the ordinary kernels reach 500 to 1290 TFLOP/s, pairs 1070 to 1540), an epilogue about six, and
-// cut tiles a launch and their partials' bytes.  So the ordinary kernels keep what fills no more than one wave of their smaller tiles
+// cut tiles a launch and their partials' bytes.  So the ordinary kernels keep small products with short K
 // (1024^3: 19.4 us against 21.5; 512 x 3072 x 2048: 27.7 against 29.7), and the last wave is cut where K is long: a weight gradient of
 // 2560 x 2048 over 8192 tokens 154 -> 66 us (uncut 92), of 1152 x 384 over 16384 132 -> 42 us (uncut 114).
 struct PairPlan { bool use; int whole, splits, kb_per_split; long long work_floats; };
 constexpr double T256 = 1.3, T128 = 0.85, EPI256 = 6.0, EPI128 = 4.0, PAIR_ITEM = 6.0, PAIR_LAUNCH = 2.0, PAIR_REDUCE = 8.0, PAIR_FLOAT = 5.6e-6;
-static PairPlan plan_pair(int M, int N, int K, int n_sm, bool may_cut) {
+static PairPlan find_pair_plan(int M, int N, int K, int n_sm, bool may_cut) {
     PairPlan best{false, 0, 1, 0, 0};
     const int pairs = n_sm / 2;
     if (M <= BM || pairs < 1) return best;
@@ -186,6 +186,16 @@ static PairPlan plan_pair(int M, int N, int K, int n_sm, bool may_cut) {
         if (c < cost) { cost = c; best = PairPlan{true, (int)whole, real, kbps, floats}; }
     }
     return best;
+}
+// A program multiplies the same few shapes over and over, and the search takes 1 to 1.5 us of host time, twice a product.
+static PairPlan plan_pair(int M, int N, int K, int n_sm, bool may_cut) {
+    struct Seen { int M, N, K, n_sm, may_cut; PairPlan plan; };
+    static thread_local Seen seen[256];          // M is 0 in an entry that holds none
+    if (M <= 0) return PairPlan{false, 0, 1, 0, 0};
+    const unsigned h = (unsigned)M * 0x9E3779B1u ^ (unsigned)N * 0x85EBCA6Bu ^ (unsigned)K * 0xC2B2AE35u ^ (unsigned)(2 * n_sm + may_cut) * 0x27D4EB2Fu;
+    Seen& e = seen[h >> 24];
+    if (e.M != M || e.N != N || e.K != K || e.n_sm != n_sm || e.may_cut != (int)may_cut) e = Seen{M, N, K, n_sm, (int)may_cut, find_pair_plan(M, N, K, n_sm, may_cut)};
+    return e.plan;
 }
 
 static int launch_pair(const void* A, long long lda, int a_mn, const void* B, long long ldb, int b_mn, void* C, long long ldc, int M, int N, int K, const float* bias,

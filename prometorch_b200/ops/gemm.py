@@ -8,6 +8,7 @@ M/N-major.  The reference's linear layers go through fp32 cublasSgemm
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import os
 from typing import Optional
 
@@ -71,6 +72,12 @@ def _sms(dev) -> int:
     return _SM_COUNT[k]
 
 
+@functools.lru_cache(maxsize=4096)
+def _work_floats(M: int, Nn: int, K: int, dev: torch.device) -> int:
+    """Floats of workspace for the partials of the last wave's tiles, where cutting them pays: a function of the shape and the device's size."""
+    return int(N.lib().ptb_gemm_work_floats(M, Nn, K, _sms(dev)))
+
+
 def _rowmajor(t):
     if t.dim() != 2 or t.stride(1) != 1:
         raise ValueError("operand must be a 2-D tensor with a contiguous last dimension")
@@ -106,11 +113,12 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
         (EPI_OUT_F32 if out.dtype == torch.float32 else 0) | (EPI_GELU if gelu else 0) | (EPI_RELU2 if relu2 else 0)
     if bias is not None:
         bias = bias.float().contiguous()
-    st = torch.cuda.current_stream(a.device).cuda_stream
-    floats = int(N.lib().ptb_gemm_work_floats(M, Nn, K, _sms(a.device)))        # partials of the last wave's tiles, where cutting them pays
-    work = torch.empty(floats, dtype=torch.float32, device=a.device) if floats else None
+    dev = a.device
+    st = torch.cuda.current_stream(dev).cuda_stream
+    floats = _work_floats(M, Nn, K, dev)
+    work = torch.empty(floats, dtype=torch.float32, device=dev) if floats else None
     N.check(N.lib().ptb_gemm_bf16_ws(a.data_ptr(), a.stride(0), int(a_mn), b.data_ptr(), b.stride(0), int(b_mn), out.data_ptr(), out.stride(0), M, Nn, K,
-                                     N.ptr(bias), flags, N.ptr(work), floats, _status(a.device).data_ptr(), 0, st), "gemm_bf16")
+                                     N.ptr(bias), flags, N.ptr(work), floats, _status(dev).data_ptr(), 0, st), "gemm_bf16")
     return out
 
 
