@@ -346,7 +346,7 @@ PTB_API int ptb_prompt_heads(void* qkv, int T, int H, int Hk, int D, const float
                              const float* sin, int neox, int pos0, void* k_cache, void* v_cache, int S, cudaStream_t st) {
     if (T <= 0) return 0;
     if (pos0 < 0 || pos0 + T > S) { ptb_set_error("prompt heads: positions %d .. %d outside a cache of %d", pos0, pos0 + T, S); return -1; }
-    if (((uintptr_t)qkv | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos | (uintptr_t)sin) & 7) { ptb_set_error("prompt heads: needs 8-byte aligned buffers"); return -1; }
+    if (((uintptr_t)qkv | (uintptr_t)q_norm | (uintptr_t)k_norm | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)cos | (uintptr_t)sin) & 7) { ptb_set_error("prompt heads: needs 8-byte aligned buffers"); return -1; }
     const long long heads = (long long)T * (H + 2 * Hk);
     auto go = [&](auto kern, int per_cta) {
         kern<<<(unsigned)((heads + per_cta - 1) / per_cta), 256, 0, st>>>((__nv_bfloat16*)qkv, heads, H, Hk, q_norm, k_norm, add_one ? 1.f : 0.f, eps, cos, sin, neox, pos0,

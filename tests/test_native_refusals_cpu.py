@@ -26,3 +26,11 @@ def test_flash_attention_delta_needs_aligned_rows(off_o, off_do, off_dq, D):
     if not off_dq:      # the backward that takes no buffer to clear
         assert "16-byte aligned" in _refused(L.ptb_flash_attn_bwd(BASE, BASE, BASE, BASE + off_o, BASE + off_do, BASE, BASE, BASE, BASE, BASE, 0, 1, 8, 8, 2, 2, D, 1,
                                                                   1.0, 0, None))
+
+
+@pytest.mark.parametrize("which", range(7))
+def test_prompt_heads_needs_aligned_operands(which):
+    """Pairs of values are read together: the projection, both norms, the tables and the caches."""
+    L = _lib()
+    a = [BASE + (4 if i == which else 0) for i in range(7)]
+    assert "8-byte aligned" in _refused(L.ptb_prompt_heads(a[0], 3, 2, 1, 64, a[1], a[2], 0, 1e-6, a[3], a[4], 1, 0, a[5], a[6], 8, None))
