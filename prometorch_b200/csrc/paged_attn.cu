@@ -187,7 +187,7 @@ struct PagedAttnParams {
     int pt_stride, n_pages;
     const __nv_bfloat16* k_pages;
     const __nv_bfloat16* v_pages;
-    float* work;                   // [B, H, nsplit, D + 2] partial (acc, max, sum) when nsplit > 1
+    float* work;                   // [B, H, nsplit, D + 2] partial (acc, max, sum) when nsplit > PA_CLUSTER
     int B, H, Hk, nsplit;
     float scale_log2;              // softmax scale times log2(e)
     int q_wide;                    // rows of q start on 16 bytes
@@ -212,7 +212,8 @@ __device__ __forceinline__ void pa_cluster_sync() { asm volatile("barrier.cluste
 // tokens, not pages, are dealt to warps: one lane per token and one warp per page had nine warps work on a request of 540 tokens
 // (per kv head of 128, groups of 4: 27 us, and 3 for the merge).  Up to sixteen splits are the CTAs of a cluster, which merge through
 // distributed shared memory; more leave partials for paged_attn_merge_kernel.
-template <int D, int G>
+// V16: the pool of values starts on 16 bytes (otherwise its values come in 4-byte pieces; as a branch in one kernel that cost 4 to 7 %).
+template <int D, int G, bool V16>
 __global__ void __launch_bounds__(PA_THREADS, G == 8 ? 1 : 2) paged_attn_decode_kernel(const __grid_constant__ PagedAttnParams P) {
     constexpr int LPT = D / 8, TPI = 32 / LPT, U = G == 8 ? 2 : 4, TG = TPI * U;
     static_assert(D == 128 || D == 64, "head size 128 or 64");
@@ -260,7 +261,11 @@ __global__ void __launch_bounds__(PA_THREADS, G == 8 ? 1 : 2) paged_attn_decode_
 #pragma unroll
         for (int u = 0; u < U; ++u) kr[u] = *reinterpret_cast<const uint4*>(P.k_pages + at + (size_t)u * TPI * D);
 #pragma unroll
-        for (int u = 0; u < U; ++u) vr[u] = *reinterpret_cast<const uint4*>(P.v_pages + at + (size_t)u * TPI * D);
+        for (int u = 0; u < U; ++u) {
+            const uint32_t* v = reinterpret_cast<const uint32_t*>(P.v_pages + at + (size_t)u * TPI * D);
+            if constexpr (V16) vr[u] = *reinterpret_cast<const uint4*>(v);
+            else vr[u] = make_uint4(v[0], v[1], v[2], v[3]);
+        }
         float s[U][G];
         {
             float kf[U][8];
@@ -396,7 +401,7 @@ __global__ void paged_attn_merge_kernel(const float* __restrict__ work, __nv_bfl
     out[((size_t)b * H + h) * D + d] = __float2bfloat16_rn(L > 0.f ? o / L : 0.f);
 }
 
-template <int D, int G>
+template <int D, int G, bool V16>
 static cudaError_t launch_decode_g(const PagedAttnParams& p, cudaStream_t st) {
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
@@ -412,7 +417,7 @@ static cudaError_t launch_decode_g(const PagedAttnParams& p, cudaStream_t st) {
     if (p.cluster) {
         static bool wide = false;
         if (p.nsplit > 8 && !wide) {
-            const cudaError_t e = cudaFuncSetAttribute(paged_attn_decode_kernel<D, G>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+            const cudaError_t e = cudaFuncSetAttribute(paged_attn_decode_kernel<D, G, V16>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             if (e != cudaSuccess) return e;
             wide = true;
         }
@@ -421,17 +426,18 @@ static cudaError_t launch_decode_g(const PagedAttnParams& p, cudaStream_t st) {
     }
     cfg.attrs = attr;
     cfg.numAttrs = n;
-    return cudaLaunchKernelEx(&cfg, paged_attn_decode_kernel<D, G>, p);
+    return cudaLaunchKernelEx(&cfg, paged_attn_decode_kernel<D, G, V16>, p);
 }
 
 template <int D>
 static int launch_decode(const PagedAttnParams& p, int G, cudaStream_t st) {
     cudaError_t e;
+    const bool v16 = !((uintptr_t)p.v_pages & 15);
     switch (G) {
-        case 1: e = launch_decode_g<D, 1>(p, st); break;
-        case 2: e = launch_decode_g<D, 2>(p, st); break;
-        case 4: e = launch_decode_g<D, 4>(p, st); break;
-        case 8: e = launch_decode_g<D, 8>(p, st); break;
+        case 1: e = v16 ? launch_decode_g<D, 1, true>(p, st) : launch_decode_g<D, 1, false>(p, st); break;
+        case 2: e = v16 ? launch_decode_g<D, 2, true>(p, st) : launch_decode_g<D, 2, false>(p, st); break;
+        case 4: e = v16 ? launch_decode_g<D, 4, true>(p, st) : launch_decode_g<D, 4, false>(p, st); break;
+        case 8: e = v16 ? launch_decode_g<D, 8, true>(p, st) : launch_decode_g<D, 8, false>(p, st); break;
         default: ptb_set_error("paged attention: group size %d not in {1, 2, 4, 8}", G); return -1;
     }
     PTB_CUDA_OK(e);
@@ -489,6 +495,7 @@ PTB_API int ptb_paged_attn_decode(const void* q, long long q_stride, void* out, 
                                   float scale, float* work, int nsplit, int* status, cudaStream_t st) {
     if (B <= 0) return 0;
     if (Hk <= 0 || H % Hk) { ptb_set_error("paged attention: %d heads over %d kv heads", H, Hk); return -1; }
+    if (((uintptr_t)k_pages & 15) || ((uintptr_t)v_pages & 3)) { ptb_set_error("paged attention: keys need a 16-byte aligned pool, values a 4-byte aligned one"); return -1; }
     if (nsplit < 1 || (nsplit > PA_CLUSTER && !work)) { ptb_set_error("paged attention: nsplit %d needs a workspace", nsplit); return -1; }
     PagedAttnParams p;
     p.q = (const __nv_bfloat16*)q; p.q_stride = q_stride; p.out = (__nv_bfloat16*)out; p.lens = lens; p.page_table = page_table;

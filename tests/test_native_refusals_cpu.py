@@ -34,3 +34,11 @@ def test_prompt_heads_needs_aligned_operands(which):
     L = _lib()
     a = [BASE + (4 if i == which else 0) for i in range(7)]
     assert "8-byte aligned" in _refused(L.ptb_prompt_heads(a[0], 3, 2, 1, 64, a[1], a[2], 0, 1e-6, a[3], a[4], 1, 0, a[5], a[6], 8, None))
+
+
+@pytest.mark.parametrize("off_k,off_v", [(8, 0), (0, 2)])
+def test_paged_attention_needs_aligned_pools(off_k, off_v):
+    """Keys are read in 16-byte pieces, values that start between them in 4-byte ones."""
+    import prometorch_b200.ops.paged  # noqa: F401
+    L = _lib()
+    assert "aligned pool" in _refused(L.ptb_paged_attn_decode(BASE, 128, BASE, 1, 2, 1, 64, BASE, BASE, 4, 4, BASE + off_k, BASE + off_v, 1.0, None, 1, BASE, None))

@@ -34,3 +34,16 @@ def test_decode_splits(G, D, nsplit):
         P.check_status(dev)
         # fp32 throughout, one rounding of the result to bf16 (2^-8 of a value) and the exponentials' 2^-21 of up to 300 weights that sum to one
         assert bool(((got.float().cpu() - want).abs() <= 2 ** -8 * want.abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("D", [64, 128])
+def test_decode_values_between_16_byte_pieces(D):
+    """A pool of values that starts four bytes into its storage gives the same result as an aligned one."""
+    from prometorch_b200.ops import paged as P
+    g = torch.Generator(device="cuda").manual_seed(D)
+    kp, vp = (torch.randn(3, 2, P.PAGE, D, device="cuda", generator=g).bfloat16() for _ in range(2))
+    off = torch.empty(vp.numel() + 2, dtype=torch.bfloat16, device="cuda")[2:].view_as(vp).copy_(vp)
+    q, table = torch.randn(1, 4 * D, device="cuda", generator=g).bfloat16(), torch.tensor([[2, 0, 1]], dtype=torch.int32, device="cuda")
+    lens = torch.tensor([150], dtype=torch.int32, device="cuda")
+    assert off.data_ptr() % 16 == 4
+    assert torch.equal(P.paged_attention_decode(q, 4, 2, D, lens, table, kp, off, nsplit=2), P.paged_attention_decode(q, 4, 2, D, lens, table, kp, vp, nsplit=2))
