@@ -831,6 +831,7 @@ static int launch_bwd(const void* q, const void* k, const void* v, const void* d
 PTB_API int ptb_flash_attn_fwd_sm100(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Tq, int Tk, int H, int Hk,
                                      int D, int causal, float scale, int q_offset, int* status, cudaStream_t st) {
     if (H % Hk) { ptb_set_error("flash attention: %d query heads over %d KV heads", H, Hk); return -1; }
+    if ((uintptr_t)o & 15) { ptb_set_error("flash attention: the output needs a 16-byte aligned base"); return -1; }
     {
         int dev = 0;
         PTB_CUDA_OK(cudaGetDevice(&dev));
@@ -851,6 +852,7 @@ PTB_API int ptb_flash_attn_fwd_sm100(const void* q, const void* k, const void* v
 PTB_API int ptb_flash_attn_varlen_fwd(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv, void* o, const int* cu, int n_seq,
                                       int max_len, long long rows, int H, int Hk, int D, int causal, float scale, int* status, cudaStream_t st) {
     if (Hk <= 0 || H % Hk) { ptb_set_error("flash attention: %d query heads over %d KV heads", H, Hk); return -1; }
+    if ((uintptr_t)o & 15) { ptb_set_error("flash attention: the output needs a 16-byte aligned base"); return -1; }
     if (!cu || rows <= 0 || n_seq <= 0) { ptb_set_error("flash attention: packed sequences need their offsets and at least one row"); return -1; }
     {
         int dev = 0;

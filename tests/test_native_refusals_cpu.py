@@ -42,3 +42,8 @@ def test_paged_attention_needs_aligned_pools(off_k, off_v):
     import prometorch_b200.ops.paged  # noqa: F401
     L = _lib()
     assert "aligned pool" in _refused(L.ptb_paged_attn_decode(BASE, 128, BASE, 1, 2, 1, 64, BASE, BASE, 4, 4, BASE + off_k, BASE + off_v, 1.0, None, 1, BASE, None))
+
+
+def test_flash_attention_output_has_to_be_aligned():
+    L = _lib()
+    assert "16-byte aligned" in _refused(L.ptb_flash_attn_varlen_fwd(BASE, 256, BASE, 256, BASE, 256, BASE + 8, BASE, 1, 4, 4, 2, 2, 64, 1, 1.0, BASE, None))
