@@ -1,8 +1,8 @@
 // FlashAttention on the 5th-generation tensor cores: both products of every 128 x 128 block run as
 // tcgen05.mma with accumulators in tensor memory, operands arrive by TMA.
 //
-// Forward: one CTA per two tiles of 128 query rows that read the same keys: the same rows of two heads of a group where the
-// group's size is even, else 256 consecutive rows of one head.  Ten warps:
+// Forward of grids that fill the GPU (others: flash_attn_tile_sm100.cuh): one CTA per two tiles of 128 query rows that read the same keys: the same rows of two
+// heads of a group where the group's size is even, else 256 consecutive rows of one head.  Ten warps:
 //   warp 8   TMA producer: both Q tiles once, then K and V tiles of 128 keys through two-stage rings;
 //   warp 9   owns tensor memory and issues the MMAs.  Tile t has 128 columns for its scores S_t and D for its output O_t; for every
 //            block j it issues, tile by tile, O_t += P_t(j) V_j and then S_t(j+1) = Q_t K_j+1^T, so that one tile's products run
@@ -43,6 +43,12 @@ struct Params {
     int units;               // CTAs per row block: B times heads (pairs of heads)
     int* status;
 };
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)), "l"(map),
+                 "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+}
 
 template <int D>
 struct Sm {
@@ -351,11 +357,64 @@ fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUte
     if (warp == 9) tmem_dealloc(tmem_base, 512);
 }
 
-// q, k, v: rows of ldq, ldk, ldv elements (heads packed along a row).
+}  // namespace fa100
+}  // namespace ptb
+
+#include "flash_attn_tile_sm100.cuh"
+
+namespace ptb {
+namespace fa100 {
+
+// Which kernel: in units of a one-tile CTA's time a two-tile CTA takes about 4/3 (1.27 to 1.5 measured where both fit the GPU at once), so what counts is the
+// waves.  One tile where it takes 3/4 of its waves or less: all grids that fit at once (1 x 4001 queries, 2 heads, size 128, causal: 63.5 us with one tile, 84.0 with
+// two; 4 x 17 over 2000 keys, 16 heads: 36.9 and 45.1), and up to 128 rows of heads without a partner, whose second tile would be empty (16 x 100, 12 heads,
+// size 64: 17.2 and 20.4).  Just past it (192 against 96 CTAs) two tiles are 0 to 41 % faster, at 512 against 256 between 18 and 62 %.
+static bool pairs_of_heads(int H, int Hk) { return (H / Hk) % 2 == 0; }         // equal lengths side by side; else neighbouring rows, one block apart at most
+static long long tile_count(int B, int Tq, int H) { return (long long)((Tq + BQ - 1) / BQ) * B * H; }
+static long long pair_count(int B, int Tq, int H, int Hk) { return pairs_of_heads(H, Hk) ? tile_count(B, Tq, H / 2) : (long long)((Tq + 2 * BQ - 1) / (2 * BQ)) * B * H; }
+static bool one_tile(int B, int Tq, int H, int Hk, int n_sm) {
+    const long long tiles = tile_count(B, Tq, H), ctas = pair_count(B, Tq, H, Hk);
+    return tiles <= 0x7fffffffLL && 3 * ((tiles + n_sm - 1) / n_sm) <= 4 * ((ctas + n_sm - 1) / n_sm);
+}
+
+// Of the current device; asked for once (the query costs the host more than the rule).
+static int sm_count() {
+    static thread_local int of = -1, n = 148;
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev != of && cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess) of = dev;
+    return n > 0 ? n : 148;
+}
+
+template <int D>
+static int launch_tile(const void* q, const void* k, const void* v, Params p, cudaStream_t st) {
+    CUtensorMap mq, mk, mv;
+    if (ptb_make_tmap_bf16_3d(&mq, q, (long long)p.H * D, p.Tq, p.B, 64, BQ, 1)) return -1;
+    if (ptb_make_tmap_bf16_3d(&mk, k, (long long)p.Hk * D, p.Tk, p.B, 64, BKV, 1)) return -1;
+    if (ptb_make_tmap_bf16_3d(&mv, v, (long long)p.Hk * D, p.Tk, p.B, 64, 64, 1)) return -1;
+    static bool attr = false;
+    if (!attr) {
+        PTB_CUDA_OK(cudaFuncSetAttribute(fwd_tile_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmTile<D>::TOTAL));
+        attr = true;
+    }
+    p.units = p.B * p.H;
+    fwd_tile_kernel<D><<<(unsigned)tile_count(p.B, p.Tq, p.H), NTHREADS, SmTile<D>::TOTAL, st>>>(mq, mk, mv, p);
+    PTB_CUDA_OK(cudaGetLastError());
+    return 0;
+}
+
+// q, k, v: rows of ldq, ldk, ldv elements (heads packed along a row; without cu rows lie next to one another).
 template <int D>
 static int launch(const void* q, long long ldq, const void* k, long long ldk, const void* v, long long ldv, void* o, float* lse, const int* cu, long long rows_q,
                   long long rows_k, int B, int Tq, int Tk, int H, int Hk, int causal, float scale, int q_offset, int* status, cudaStream_t st) {
     if (B <= 0 || Tq <= 0 || H <= 0) return 0;
+    Params p;
+    p.O = (__nv_bfloat16*)o; p.lse = lse; p.cu = cu; p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
+    p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
+    p.pair_heads = pairs_of_heads(H, Hk);
+    p.units = B * (p.pair_heads ? H / 2 : H);
+    const long long ctas = pair_count(B, Tq, H, Hk);
+    if (ctas > 0x7fffffffLL) { ptb_set_error("flash attention: %lld tiles", ctas); return -1; }
+    if (!cu && one_tile(B, Tq, H, Hk, sm_count())) return launch_tile<D>(q, k, v, p, st);
     CUtensorMap mq, mk, mv;
     if (ptb_make_tmap_bf16(&mq, q, (long long)H * D, rows_q, ldq, 64, BQ)) return -1;
     if (ptb_make_tmap_bf16(&mk, k, (long long)Hk * D, rows_k, ldk, 64, BKV)) return -1;
@@ -365,14 +424,6 @@ static int launch(const void* q, long long ldq, const void* k, long long ldk, co
         PTB_CUDA_OK(cudaFuncSetAttribute(fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, Sm<D>::TOTAL));
         attr = true;
     }
-    Params p;
-    p.O = (__nv_bfloat16*)o; p.lse = lse; p.cu = cu; p.B = B; p.Tq = Tq; p.Tk = Tk; p.H = H; p.Hk = Hk; p.causal = causal; p.q_offset = q_offset;
-    p.scale_log2 = scale * 1.4426950408889634f; p.status = status;
-    p.pair_heads = (H / Hk) % 2 == 0;                 // equal lengths side by side; else neighbouring rows, one block apart at most
-    p.units = B * (p.pair_heads ? H / 2 : H);
-    const int rows = p.pair_heads ? BQ : 2 * BQ;
-    const long long ctas = (long long)((Tq + rows - 1) / rows) * p.units;
-    if (ctas > 0x7fffffffLL) { ptb_set_error("flash attention: %lld tiles", ctas); return -1; }
     fwd_kernel<D><<<(unsigned)ctas, NTHREADS, Sm<D>::TOTAL, st>>>(mq, mk, mv, p);
     PTB_CUDA_OK(cudaGetLastError());
     return 0;
@@ -438,11 +489,6 @@ struct SmB {
     static_assert(TOTAL <= 232448, "shared memory of one CTA");
 };
 
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int c0, int c1, int c2, uint64_t* bar) {
-    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)), "l"(map),
-                 "r"(smem_u32(bar)), "r"(c0), "r"(c1), "r"(c2)
-                 : "memory");
-}
 __device__ __forceinline__ void tma_reduce_add_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1),
                  "r"(c2)
@@ -846,6 +892,9 @@ PTB_API int ptb_flash_attn_fwd_sm100(const void* q, const void* k, const void* v
     ptb_set_error("flash attention (tcgen05): head size %d not supported (64, 128)", D);
     return -1;
 }
+
+// Whether the forward of these sizes runs one tile of 128 rows per CTA on a GPU of n_sm SMs (packed sequences never do).
+PTB_API int ptb_flash_attn_one_tile(int B, int Tq, int H, int Hk, int n_sm) { return ptb::fa100::one_tile(B, Tq, H, Hk, n_sm); }
 
 // Sequences of different lengths packed by rows: sequence i has rows cu[i] .. cu[i + 1] (cu: device int [n_seq + 1], rows in all, none longer
 // than max_len) of q, k and v, whose rows are ldq, ldk and ldv elements apart with the heads packed along them; o [rows, H, D].  One launch.

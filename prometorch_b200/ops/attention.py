@@ -1,10 +1,10 @@
 """Attention front end: ``flash_attention(q, k, v, causal)`` on ``[B, T, heads, D]`` tensors with
 grouped-query heads (``heads_q`` a multiple of ``heads_kv``).
 
-CUDA bf16 inputs with D in {64, 128} run the hand-written FlashAttention kernels: the forward on
-tcgen05 tensor cores with TMEM accumulators and TMA-fed tiles (csrc/flash_attn_sm100.cu; it also returns the
-log-sum-exp), the recompute-based backward with the GQA reduction of dK/dV done inside the kernel
-(csrc/flash_attn.cu, which also holds an mma.sync forward selected by PTB_FA_SM100=0).  ``q_offset`` /
+CUDA bf16 inputs with D in {64, 128} run the hand-written FlashAttention kernels on tcgen05 tensor cores with TMEM
+accumulators and TMA-fed tiles (csrc/flash_attn_sm100.cu): the forward, which also returns the log-sum-exp, and the
+recompute-based backward with the GQA reduction of dK/dV done inside the kernel.  csrc/flash_attn.cu has the backward's row term
+and the mma.sync kernels that PTB_FA_SM100=0 and PTB_FA_BWD_SM100=0 select.  ``q_offset`` /
 ``return_lse`` are the hooks a ring/context-parallel wrapper needs: blocks of K/V can be processed
 separately and merged by log-sum-exp.  CPU tensors use the plain softmax formulation.  The layout
 matches the reference's kernel, which also takes ``[B, N, H, D]`` (aten/src/ATen/native/Attention.h:244-250)."""
@@ -34,6 +34,8 @@ def _decls(L):
         L.ptb_flash_attn_bwd_sm100.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, ci, ci, ci, ci, ci, ci, ci, cf, ci, ci, vp, vp]
         L.ptb_flash_attn_bwd_sm100.restype = ci
     ll = C.c_longlong
+    L.ptb_flash_attn_one_tile.argtypes = [ci] * 5
+    L.ptb_flash_attn_one_tile.restype = ci
     L.ptb_flash_attn_varlen_fwd.argtypes = [vp, ll, vp, ll, vp, ll, vp, vp, ci, ci, ll, ci, ci, ci, ci, cf, vp, vp]
     L.ptb_flash_attn_varlen_fwd.restype = ci
 

@@ -16,11 +16,21 @@ SHAPES = [(1, 1, 1, 2, 1, 64, True, 0), (1, 127, 127, 2, 2, 128, True, 0), (2, 1
           (1, 640, 640, 5, 5, 128, True, 0)]
 
 
+def _one_tile(B, Tq, H, Hk):
+    from prometorch_b200 import _native as N
+    return bool(N.lib().ptb_flash_attn_one_tile(B, Tq, H, Hk, torch.cuda.get_device_properties(0).multi_processor_count))
+
+
 @pytest.mark.parametrize("B,Tq,Tk,H,Hk,D,causal,off", SHAPES)
 @pytest.mark.parametrize("scale", [None, 3.0])
-def test_forward_tiles(B, Tq, Tk, H, Hk, D, causal, off, scale):
-    """``scale`` 3: maxima that keep growing from block to block, so that outputs are scaled on the way."""
+@pytest.mark.parametrize("full", [False, True])
+def test_forward_tiles(B, Tq, Tk, H, Hk, D, causal, off, scale, full):
+    """``scale`` 3: maxima that keep growing from block to block, so that outputs are scaled on the way.  ``full``: as many entries as give every
+    SM a tile and more, which takes the kernel with two tiles a CTA; fewer take the one with one, as do rows whose second tile would be empty."""
     from prometorch_b200.ops.attention import attention_reference, flash_attention
+    if full:
+        B = -(-160 // (-(-Tq // 128) * H))
+    assert _one_tile(B, Tq, H, Hk) == (not full or (Tq <= 128 and (H // Hk) % 2 == 1))
     g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
     q, k, v = (torch.randn(B, t, h, D, device="cuda", generator=g).bfloat16() for t, h in ((Tq, H), (Tk, Hk), (Tk, Hk)))
     if scale:
@@ -76,7 +86,8 @@ def test_backward_tiles(B, Tq, Tk, H, Hk, D, causal, off):
 
 @pytest.mark.parametrize("Tq,Tk,causal", [(129, 129, True), (130, 70, False), (1, 257, False)])
 @pytest.mark.parametrize("D", [64, 128])
-def test_entries_of_a_batch_stay_apart(Tq, Tk, causal, D):
+@pytest.mark.parametrize("entries", [2, 40])
+def test_entries_of_a_batch_stay_apart(Tq, Tk, causal, D, entries):
     """Ragged last blocks lie over the next entry's rows: what is not finite there reaches neither outputs nor gradients of the entry before."""
     from prometorch_b200.ops.attention import flash_attention
     g = torch.Generator(device="cuda").manual_seed(Tq + Tk)
@@ -88,17 +99,19 @@ def test_entries_of_a_batch_stay_apart(Tq, Tk, causal, D):
         return [o.detach(), *torch.autograd.grad(o, (q, k, v), x[3])]
     want = run(one)
     for bad in (float("inf"), float("nan")):
-        got = run([torch.cat([t, torch.full_like(t, bad)]) for t in one])
+        got = run([torch.cat([t, torch.full_like(t, bad)] * (entries // 2)) for t in one])
         for a, b in zip(got, want):             # the order in which key blocks are added to dQ is free
-            assert bool(torch.isfinite(a[0]).all()) and _rel(a[0], b[0].double()) < 1e-3
+            assert bool(torch.isfinite(a[::2]).all()) and _rel(a[::2], b.double().expand_as(a[::2])) < 1e-3
 
 
 @pytest.mark.parametrize("peak", [1.0, 3.0])
 @pytest.mark.parametrize("D", [64, 128])
-def test_forward_error_is_that_of_exact_maxima(peak, D):
+@pytest.mark.parametrize("H", [2, 24])
+def test_forward_error_is_that_of_exact_maxima(peak, D, H):
     """Weights are rounded to bf16 under the running maximum of each block: no further from 64 bits than the same roundings in 64-bit arithmetic."""
     from prometorch_b200.ops.attention import flash_attention
-    T, H, two = 1025, 2, 1.4426950408889634
+    T, two = 1025, 1.4426950408889634
+    assert _one_tile(1, T, H, H) == (H == 2)
     g = torch.Generator(device="cuda").manual_seed(D)
     q, k, v = ((torch.randn(T, H, D, device="cuda", generator=g) * s).bfloat16() for s in (peak, 1, 1))
     o = flash_attention(q[None], k[None], v[None], causal=True)[0]
