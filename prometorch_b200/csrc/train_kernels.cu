@@ -9,6 +9,7 @@
 // access, keeps a row in registers between its reduction and its update, and
 // touches HBM once per operand.
 #include "common.cuh"
+#include <type_traits>
 
 namespace ptb {
 
@@ -809,16 +810,15 @@ PTB_API int ptb_rmsnorm_fwd(const void* x, const void* w, void* y, float* rstd, 
 template <typename T>
 static void launch_rmsnorm_bwd(const void* x, const void* w, const void* dy, const float* rstd, void* dx, void* dw, float* dw_partial,
                                int n_ctas, long long rows, int H, const void* dresid, cudaStream_t st) {
-    using B = __nv_bfloat16;
-    auto wide = [&](auto kern) { kern<<<n_ctas, 256, 0, st>>>((const B*)x, (const B*)w, (const B*)dy, rstd, (B*)dx, dw_partial, rows, H, (const B*)dresid); };
-    if (sizeof(T) == 2 && H > 1024 && H <= 2048) wide(rmsnorm_bwd_wide_kernel<2>);
-    else if (sizeof(T) == 2 && H > 2048 && H <= 4096) wide(rmsnorm_bwd_wide_kernel<4>);
-    else if (H <= 2048) {
-        rmsnorm_bwd_warp_kernel<T, 8><<<n_ctas, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, (const T*)dresid);
-    } else if (H <= 4096) {
-        rmsnorm_bwd_warp_kernel<T, 16><<<n_ctas, 256, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, (const T*)dresid);
+    auto go = [&](auto kern, int threads) { kern<<<n_ctas, threads, 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, rows, H, (const T*)dresid); };
+    if (H > 4096) go(rmsnorm_bwd_kernel<T>, rms_threads(H));
+    else if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+        if (H > 2048) go(rmsnorm_bwd_wide_kernel<4>, 256);
+        else if (H > 1024) go(rmsnorm_bwd_wide_kernel<2>, 256);
+        else go(rmsnorm_bwd_warp_kernel<T, 8>, 256);
     } else {
-        rmsnorm_bwd_kernel<T><<<n_ctas, rms_threads(H), 0, st>>>((const T*)x, (const T*)w, (const T*)dy, rstd, (T*)dx, dw_partial, (int)rows, H, (const T*)dresid);
+        if (H > 2048) go(rmsnorm_bwd_warp_kernel<T, 16>, 256);
+        else go(rmsnorm_bwd_warp_kernel<T, 8>, 256);
     }
     colsum2_kernel<T><<<(H + 31) / 32, 256, 0, st>>>(dw_partial, n_ctas, H, (T*)dw);
 }
