@@ -39,7 +39,7 @@ class FusedLayerNorm(nn.LayerNorm):
 
     The kernel saves the GPU about 15 us per million values (16384 x 384: 132 us forward and backward with torch's op, 38 here; 4096 x 384: 48
     and 26), but as a Python function it costs the host 46 us more than torch's op.  Up to ``LARGE`` values the host is what bounds a step
-    of the models that use it (four 384-wide layers, 16384 tokens: 5.5 ms of host work beside 4.8 of GPU work with torch's op)."""
+    of the models that use it (four 384-wide layers, 16384 tokens: 5.5 ms of host work beside 4.6 of GPU work with torch's op)."""
     LARGE = 1 << 23
 
     def forward(self, x):
